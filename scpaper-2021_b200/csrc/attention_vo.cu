@@ -2,16 +2,26 @@
 //   out[t, :] = bias_o + sum_h softmax(scale * Q_h K_h^T + mask)[t, :] . VO_h
 // where VO[b][h] = X_b W_VO[h] has the full model width.
 //
-// One CTA owns 128 queries of one sequence and a chunk of up to 256 output features, whose
-// fp32 accumulator lives in tensor memory for the whole kernel: heads are reduced inside the
-// accumulator in a fixed order (h = 0, 1, ...), so the result is deterministic and the output
-// needs no pre-zeroing (the reference reduces heads with half2 atomics).  Because every
-// head has its own softmax normaliser, probabilities are normalised BEFORE the second
-// product: for sequences longer than one key block a first pass over the head's key blocks
-// computes the row max and sum (scores only), a second pass recomputes the scores, writes
-// P = exp2(s - m) / l as the fp16 A operand and accumulates O += P . VO_h[block].
-// Roles, TMA layouts and bounded waits are those of attention.cu.
+// A work item is 128 queries of one sequence and a chunk of up to 256 output features.  Its heads
+// are dealt to the CTAs of a thread-block cluster (contiguous ranges; one CTA when the items alone
+// fill the machine).  A CTA accumulates its heads' O += P_h . VO_h in tensor memory, in the order
+// of the heads; at the end the cluster's partial sums meet in distributed shared memory, every CTA
+// adding the ranks' contributions to its share of the rows in rank order, so the result is
+// deterministic and the output needs no pre-zeroing (the reference reduces heads with half2
+// atomics).  Because every head has its own softmax normaliser, probabilities are normalised
+// BEFORE the second product: for sequences longer than one key block a first pass over the head's
+// key blocks computes the row max and sum (scores only), a second pass recomputes the scores,
+// writes P = exp2(s - m) / l as the fp16 A operand and accumulates O += P . VO_h[block].
+//
+// What bounds it: per head and key block the tensor core needs 1280 cycles (256 for the scores,
+// 1024 for 128 x 256 x 128) and the special-function unit 1024 (128 x 128 exponentials), so the
+// kernel is a pipeline of the two: two score buffers in tensor memory (S of the next task is
+// computed while this task's softmax runs), probabilities held in registers until the previous
+// P . VO has left the P tile, Q / K of the next task and VO in half blocks of 64 keys prefetched
+// by two producer warps.
 #include <math.h>
+
+#include <type_traits>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -21,13 +31,35 @@ namespace {
 
 constexpr int BQ = 128;
 constexpr int BKV = 128;
-constexpr int VO_THREADS = 192;
+constexpr int VO_KEYS = 64;                        // keys of one VO stage
+constexpr int VO_STAGES = 3;
+constexpr int VO_SM_WARPS = 8;                     // softmax / output warps
+constexpr int VO_SM_THREADS = 32 * VO_SM_WARPS;
+constexpr int VO_THREADS = 96 + VO_SM_THREADS;     // + Q/K producer, MMA issuer, VO producer
+constexpr int VO_MAX_CLUSTER = 8;
 constexpr int ATOM_BYTES = 128 * 128;
-// NC output features per CTA: 256, or 128 / 64 behind a test hook.  A CTA recomputes the scores
-// and the softmax of every head whatever its width, so narrower chunks do more work in total
-// and spread it over more CTAs.  Tensor memory: scores in columns [0, 128), the accumulator
-// behind them.
-__host__ __device__ constexpr int vo_tmem_cols(int nc) { return nc <= 128 ? 256 : 512; }
+constexpr int VO_ATOM = VO_KEYS * 128;             // 64 keys x 64 features
+constexpr int VO_QK_BYTES = 4 * ATOM_BYTES;        // two stages of 64-wide heads or one of 128-wide
+// NC output features per CTA: 256, or 128 / 64 behind a test hook.  Tensor memory: two score
+// buffers in columns [0, 256), the accumulator behind them.
+constexpr int VO_TMEM_COLS = 512;
+__host__ __device__ constexpr int vo_stage_bytes(int nc) { return (nc / 64) * VO_ATOM; }
+// fp32 rows of the final exchange, padded so that a warp's 16-byte stores (one row per lane) hit
+// all banks
+__host__ __device__ constexpr int vo_pitch(int nc) { return nc * 4 + 16; }
+__host__ __device__ constexpr int vo_exchange_bytes(int nc, int csize) {
+    return csize * ((BQ + csize - 1) / csize) * vo_pitch(nc);
+}
+__host__ __device__ constexpr int vo_smem_bytes(int nc) {
+    // the exchange overlays the operand stages once the last product is complete
+    const int operands = VO_QK_BYTES + VO_STAGES * vo_stage_bytes(nc);
+    int exchange = 0;
+    for (int g = 1; g <= VO_MAX_CLUSTER; ++g)
+        exchange = vo_exchange_bytes(nc, g) > exchange ? vo_exchange_bytes(nc, g) : exchange;
+    return (operands > exchange ? (operands + 1023) / 1024 * 1024 : (exchange + 1023) / 1024 * 1024) +
+           2 * ATOM_BYTES + 256 + 4 * BQ * 4 + 1024;
+}
+static_assert(vo_smem_bytes(256) <= 227 * 1024, "shared memory budget exceeded");
 
 struct VoArgs {
     __half* out;
@@ -35,13 +67,24 @@ struct VoArgs {
     const __half* mask;
     const int* valid_len;
     int batch, seq, nhead, dh_qk, emdim;
-    int mask_kind;
     float scale_log2;
     int* err_word;
 };
 
-template <int NC>
-__global__ void __launch_bounds__(VO_THREADS, (NC <= 128 ? 2 : 1))
+__device__ __forceinline__ uint32_t vo_cluster_size() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void st_cluster_v4(uint32_t addr, uint32_t x, uint32_t y, uint32_t z,
+                                              uint32_t w) {
+    asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(x), "r"(y),
+                 "r"(z), "r"(w)
+                 : "memory");
+}
+
+template <int NC, int MASK>
+__global__ void __launch_bounds__(VO_THREADS, 1)
 attention_vo_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                     const __grid_constant__ CUtensorMap tmVO, const VoArgs a) {
     extern __shared__ uint8_t smem_raw[];
@@ -49,313 +92,395 @@ attention_vo_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     // shared-memory provenance (plain LDS / STS instead of generic accesses)
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     const int nqa = (a.dh_qk + 63) >> 6;
-    uint8_t* sQ = smem;
-    uint8_t* sK = sQ + nqa * ATOM_BYTES;
-    uint8_t* sVO = sK + nqa * ATOM_BYTES;
-    uint8_t* sP = sVO + (NC / 64) * ATOM_BYTES;
+    const int qk_stages = nqa == 1 ? 2 : 1;
+    const int qk_stage_bytes = 2 * nqa * ATOM_BYTES;
+    uint8_t* sQK = smem;
+    uint8_t* sVO = sQK + VO_QK_BYTES;
+    uint8_t* sP = smem + vo_smem_bytes(NC) - 1024 - (2 * ATOM_BYTES + 256 + 4 * BQ * 4);
     uint64_t* bars = reinterpret_cast<uint64_t*>(sP + 2 * ATOM_BYTES);
-    uint64_t* qk_full = bars + 0;
-    uint64_t* qk_empty = bars + 1;
-    uint64_t* vo_full = bars + 2;
-    uint64_t* vo_empty = bars + 3;
-    uint64_t* s_full = bars + 4;
-    uint64_t* s_free = bars + 5;
-    uint64_t* p_full = bars + 6;
-    uint64_t* pv_done = bars + 7;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
+    uint64_t* qk_full = bars;        // [2]
+    uint64_t* qk_empty = bars + 2;   // [2]
+    uint64_t* vo_full = bars + 4;    // [VO_STAGES]
+    uint64_t* vo_empty = bars + 7;   // [VO_STAGES]
+    uint64_t* s_full = bars + 10;    // [2]
+    uint64_t* s_free = bars + 12;    // [2]
+    uint64_t* p_full = bars + 14;
+    uint64_t* pv_done = bars + 15;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    float* s_x = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + 256);  // [2][2][128]
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
-    const int q0 = blockIdx.x * BQ;
+    const int csize = static_cast<int>(vo_cluster_size());
+    const int rank = static_cast<int>(cluster_ctarank());
+    const int q0 = static_cast<int>(blockIdx.x / csize) * BQ;
     const int e0 = blockIdx.y * NC;
     const int b = blockIdx.z;
     const int n_c = (a.emdim - e0) < NC ? (a.emdim - e0) : NC;  // multiple of 16
     const int nca = (n_c + 63) >> 6;
-
-    int kv_len = a.seq;
-    if (a.mask_kind == ET_MASK_PADDING) {
-        kv_len = a.valid_len[b];
-        kv_len = kv_len < 0 ? 0 : (kv_len > a.seq ? a.seq : kv_len);
-    }
-    int n_kv = (kv_len + BKV - 1) / BKV;
-    if (a.mask_kind == ET_MASK_CAUSAL) {
-        const int last_q = (q0 + BQ - 1 < a.seq ? q0 + BQ - 1 : a.seq - 1);
-        const int lim = last_q / BKV + 1;
-        n_kv = n_kv < lim ? n_kv : lim;
-    }
-    const int passes = n_kv > 1 ? 2 : 1;  // statistics pass only when a row spans several blocks
+    const int h_begin = a.nhead * rank / csize, h_end = a.nhead * (rank + 1) / csize;
 
     if (threadIdx.x == 0) {
-        mbar_init(qk_full, 1);
-        mbar_init(qk_empty, 1);
-        mbar_init(vo_full, 1);
-        mbar_init(vo_empty, 1);
-        mbar_init(s_full, 1);
-        mbar_init(s_free, 128);
-        mbar_init(p_full, 128);
+        tma_prefetch_desc(&tmQ);
+        tma_prefetch_desc(&tmK);
+        tma_prefetch_desc(&tmVO);
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&qk_full[i], 1);
+            mbar_init(&qk_empty[i], 1);
+            mbar_init(&s_full[i], 1);
+            mbar_init(&s_free[i], VO_SM_THREADS);
+        }
+        for (int i = 0; i < VO_STAGES; ++i) {
+            mbar_init(&vo_full[i], 1);
+            mbar_init(&vo_empty[i], 1);
+        }
+        mbar_init(p_full, VO_SM_THREADS);
         mbar_init(pv_done, 1);
         *abort_flag = 0;
         fence_barrier_init();
     }
     if (warp == 1) {
-        tmem_alloc(tmem_slot, vo_tmem_cols(NC));
+        tmem_alloc(tmem_slot, VO_TMEM_COLS);
         tmem_relinquish();
     }
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
-    const uint32_t tmem_S = tmem_base;
-    const uint32_t tmem_O = tmem_base + 128;
+    const uint32_t tmem_O = tmem_base + 256;
     pdl_launch_dependents();
     pdl_wait();  // every input is produced by earlier kernels on the stream
 
+    int kv_len = a.seq;
+    if (MASK == ET_MASK_PADDING) {
+        kv_len = __ldcg(a.valid_len + b);
+        kv_len = kv_len < 0 ? 0 : (kv_len > a.seq ? a.seq : kv_len);
+    }
+    int n_kv = (kv_len + BKV - 1) / BKV;
+    if (MASK == ET_MASK_CAUSAL) {
+        const int last_q = (q0 + BQ - 1 < a.seq ? q0 + BQ - 1 : a.seq - 1);
+        const int lim = last_q / BKV + 1;
+        n_kv = n_kv < lim ? n_kv : lim;
+    }
+    const int passes = n_kv > 1 ? 2 : 1;  // statistics pass only when a row spans several blocks
+    // Task t of this CTA: (head, pass, key block), in that order of nesting.
+    const int per_head = passes * n_kv;
+    const int n_task = (h_end - h_begin) * per_head;
+
     if (warp == 0) {
-        // ---------------- TMA producer ----------------
-        if (n_kv > 0 && elect_one()) {
-            tma_prefetch_desc(&tmQ);
-            tma_prefetch_desc(&tmK);
-            tma_prefetch_desc(&tmVO);
-            int t_qk = 0, t_vo = 0;
-            bool ok = true;
-            for (int h = 0; ok && h < a.nhead; ++h)
-                for (int pass = 0; ok && pass < passes; ++pass)
-                    for (int j = 0; ok && j < n_kv; ++j) {
-                        ok = mbar_wait_bounded(qk_empty, (t_qk & 1) ^ 1, abort_flag);
-                        if (!ok) break;
-                        mbar_arrive_expect_tx(qk_full, 2 * nqa * ATOM_BYTES);
-                        for (int t = 0; t < nqa; ++t) {
-                            tma_load_3d(sQ + t * ATOM_BYTES, &tmQ, qk_full, h * a.dh_qk + t * 64, q0, b);
-                            tma_load_3d(sK + t * ATOM_BYTES, &tmK, qk_full, h * a.dh_qk + t * 64,
-                                        j * BKV, b);
-                        }
-                        ++t_qk;
-                        if (pass == passes - 1) {
-                            ok = mbar_wait_bounded(vo_empty, (t_vo & 1) ^ 1, abort_flag);
-                            if (!ok) break;
-                            mbar_arrive_expect_tx(vo_full, nca * ATOM_BYTES);
-                            for (int t = 0; t < nca; ++t)
-                                tma_load_3d(sVO + t * ATOM_BYTES, &tmVO, vo_full, e0 + t * 64, j * BKV,
-                                            b * a.nhead + h);
-                            ++t_vo;
-                        }
-                    }
-            if (!ok) report_error(a.err_word, abort_flag, DEV_TIMEOUT_VO_PRODUCER);
-            if (*abort_flag) {
-                if (t_qk > 0)
-                    for (uint32_t it = 0; it < ET_SPIN_LIMIT; ++it)
-                        if (mbar_try_wait(qk_full, (t_qk - 1) & 1)) break;
-                if (t_vo > 0)
-                    for (uint32_t it = 0; it < ET_SPIN_LIMIT; ++it)
-                        if (mbar_try_wait(vo_full, (t_vo - 1) & 1)) break;
+        // ---------------- Q / K producer ----------------
+        if (n_task > 0 && elect_one()) {
+            int h = h_begin, in_head = 0, t = 0;
+            for (; t < n_task; ++t) {
+                const int s = t % qk_stages;
+                if (!mbar_wait_bounded(&qk_empty[s], ((t / qk_stages) & 1) ^ 1, abort_flag)) {
+                    report_error(a.err_word, abort_flag, DEV_TIMEOUT_VO_PRODUCER);
+                    break;
+                }
+                const int j = in_head >= n_kv ? in_head - n_kv : in_head;
+                uint8_t* st = sQK + s * qk_stage_bytes;
+                mbar_arrive_expect_tx(&qk_full[s], qk_stage_bytes);
+                for (int i = 0; i < nqa; ++i) {
+                    tma_load_3d(st + i * ATOM_BYTES, &tmQ, &qk_full[s], h * a.dh_qk + i * 64, q0, b);
+                    tma_load_3d(st + (nqa + i) * ATOM_BYTES, &tmK, &qk_full[s], h * a.dh_qk + i * 64,
+                                j * BKV, b);
+                }
+                if (++in_head == per_head) {
+                    in_head = 0;
+                    ++h;
+                }
             }
+            if (*abort_flag)  // let copies in flight land before shared memory is released
+                for (int i = t > qk_stages ? t - qk_stages : 0; i < t; ++i)
+                    for (uint32_t it = 0; it < ET_SPIN_LIMIT; ++it)
+                        if (mbar_try_wait(&qk_full[i % qk_stages], (i / qk_stages) & 1)) break;
+        }
+    } else if (warp == 2) {
+        // ---------------- VO producer: half blocks of 64 keys ----------------
+        if (n_task > 0 && elect_one()) {
+            const int halves = 2 * n_kv;
+            const int total = (h_end - h_begin) * halves;
+            int h = h_begin, in_head = 0, i = 0;
+            for (; i < total; ++i) {
+                const int s = i % VO_STAGES;
+                if (!mbar_wait_bounded_relaxed(&vo_empty[s], ((i / VO_STAGES) & 1) ^ 1, abort_flag)) {
+                    report_error(a.err_word, abort_flag, DEV_TIMEOUT_VO_PRODUCER);
+                    break;
+                }
+                mbar_arrive_expect_tx(&vo_full[s], nca * VO_ATOM);
+                for (int c = 0; c < nca; ++c)
+                    tma_load_3d(sVO + s * vo_stage_bytes(NC) + c * VO_ATOM, &tmVO, &vo_full[s],
+                                e0 + c * 64, in_head * VO_KEYS, b * a.nhead + h);
+                if (++in_head == halves) {
+                    in_head = 0;
+                    ++h;
+                }
+            }
+            if (*abort_flag)
+                for (int k = i > VO_STAGES ? i - VO_STAGES : 0; k < i; ++k)
+                    for (uint32_t it = 0; it < ET_SPIN_LIMIT; ++it)
+                        if (mbar_try_wait(&vo_full[k % VO_STAGES], (k / VO_STAGES) & 1)) break;
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (n_kv > 0 && elect_one()) {
+        if (n_task > 0 && elect_one()) {
             const uint32_t idesc_s = make_idesc_f16(BQ, BKV, 0, 0);
-            const uint32_t idesc_o = make_idesc_f16(BQ, n_c, 0, 1);
-            const uint32_t q_addr = smem_u32(sQ), k_addr = smem_u32(sK), vo_addr = smem_u32(sVO),
-                           p_addr = smem_u32(sP);
-            int t_s = 0, t_b = 0;
-            bool ok = true;
-            for (int h = 0; ok && h < a.nhead; ++h)
-                for (int pass = 0; ok && pass < passes; ++pass)
-                    for (int j = 0; ok && j < n_kv; ++j) {
-                        ok = mbar_wait_bounded(qk_full, t_s & 1, abort_flag) &&
-                             mbar_wait_bounded(s_free, (t_s & 1) ^ 1, abort_flag);
+            const uint32_t idesc_o = make_idesc_f16(BQ, n_c, 0, 1);  // VO is MN-major
+            const uint32_t qk_addr = smem_u32(sQK), vo_addr = smem_u32(sVO), p_addr = smem_u32(sP);
+            auto issue_s = [&](int t) -> bool {
+                const int s = t % qk_stages;
+                if (!mbar_wait_bounded(&qk_full[s], (t / qk_stages) & 1, abort_flag) ||
+                    !mbar_wait_bounded(&s_free[t & 1], ((t >> 1) & 1) ^ 1, abort_flag))
+                    return false;
+                tc_fence_after_sync();
+                const uint32_t q_addr = qk_addr + s * qk_stage_bytes;
+                const uint32_t k_addr = q_addr + nqa * ATOM_BYTES;
+                for (int kk = 0; kk < (a.dh_qk >> 4); ++kk) {
+                    const uint32_t off = (kk >> 2) * ATOM_BYTES + (kk & 3) * 32;
+                    mma_f16_ss(tmem_base + (t & 1) * BKV, make_smem_desc(q_addr + off, 16, 1024, SWZ_128B),
+                               make_smem_desc(k_addr + off, 16, 1024, SWZ_128B), idesc_s,
+                               kk != 0 ? 1u : 0u);
+                }
+                mma_commit(&s_full[t & 1]);
+                mma_commit(&qk_empty[s]);
+                return true;
+            };
+            bool ok = issue_s(0);
+            int in_head = 0, t_b = 0, v = 0;
+            for (int t = 0; ok && t < n_task; ++t) {
+                if (t + 1 < n_task) ok = issue_s(t + 1);
+                if (!ok) break;
+                if (in_head >= per_head - n_kv) {
+                    ok = mbar_wait_bounded(p_full, t_b & 1, abort_flag);
+                    for (int half = 0; ok && half < 2; ++half, ++v) {
+                        const int s = v % VO_STAGES;
+                        ok = mbar_wait_bounded(&vo_full[s], (v / VO_STAGES) & 1, abort_flag);
                         if (!ok) break;
                         tc_fence_after_sync();
-                        for (int kk = 0; kk < (a.dh_qk >> 4); ++kk) {
-                            const uint32_t off = (kk >> 2) * ATOM_BYTES + (kk & 3) * 32;
-                            mma_f16_ss(tmem_S, make_smem_desc(q_addr + off, 16, 1024, SWZ_128B),
-                                       make_smem_desc(k_addr + off, 16, 1024, SWZ_128B), idesc_s,
-                                       kk != 0 ? 1u : 0u);
-                        }
-                        mma_commit(s_full);
-                        mma_commit(qk_empty);
-                        ++t_s;
-                        if (pass == passes - 1) {
-                            ok = mbar_wait_bounded(p_full, t_b & 1, abort_flag) &&
-                                 mbar_wait_bounded(vo_full, t_b & 1, abort_flag);
-                            if (!ok) break;
-                            tc_fence_after_sync();
+                        const uint32_t vb = vo_addr + s * vo_stage_bytes(NC);
 #pragma unroll
-                            for (int kk = 0; kk < BKV / 16; ++kk) {
-                                const uint32_t p_off = (kk >> 2) * ATOM_BYTES + (kk & 3) * 32;
-                                mma_f16_ss(tmem_O,
-                                           make_smem_desc(p_addr + p_off, 16, 1024, SWZ_128B),
-                                           make_smem_desc(vo_addr + kk * 2048, ATOM_BYTES, 1024,
-                                                          SWZ_128B),
-                                           idesc_o, (t_b | kk) != 0 ? 1u : 0u);
-                            }
-                            mma_commit(pv_done);
-                            mma_commit(vo_empty);
-                            ++t_b;
-                        }
+                        for (int kk = 0; kk < VO_KEYS / 16; ++kk)
+                            mma_f16_ss(tmem_O,
+                                       make_smem_desc(p_addr + half * ATOM_BYTES + kk * 32, 16, 1024, SWZ_128B),
+                                       make_smem_desc(vb + kk * 2048, VO_ATOM, 1024, SWZ_128B), idesc_o,
+                                       (t_b | half | kk) != 0 ? 1u : 0u);
+                        mma_commit(&vo_empty[s]);
                     }
+                    if (!ok) break;
+                    mma_commit(pv_done);
+                    ++t_b;
+                }
+                if (++in_head == per_head) in_head = 0;
+            }
             if (!ok) report_error(a.err_word, abort_flag, DEV_TIMEOUT_VO_MMA);
         }
     } else {
-        // ---------------- softmax / output warps ----------------
+        // ---------------- softmax warps: two per quadrant, 64 keys of a query row each --------
         const int qd = warp & 3;
+        const int hf = (warp - 3) >> 2;
         const int r = qd * 32 + lane;
         const int qrow = q0 + r;
         const uint32_t lane_off = static_cast<uint32_t>(qd * 32) << 16;
         const float NINF = -INFINITY;
-        const __half* mrow = (a.mask_kind == ET_MASK_ADDITIVE && qrow < a.seq)
+        float* x_a = s_x;           // [2 halves][128 rows]: maxima
+        float* x_b = s_x + 2 * BQ;  // [2 halves][128 rows]: sums
+        const __half* mrow = (MASK == ET_MASK_ADDITIVE && qrow < a.seq)
                                  ? a.mask + static_cast<size_t>(qrow) * a.seq
                                  : nullptr;
-        int t_s = 0, t_b = 0;
+        auto pair_sync = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(2 + qd) : "memory"); };
+        int t = 0, t_b = 0;
         bool ok = true;
 
-        auto score = [&](uint32_t raw, int kc) -> float {
-            if (kc >= kv_len || (a.mask_kind == ET_MASK_CAUSAL && kc > qrow)) return NINF;
-            float s = __uint_as_float(raw) * a.scale_log2;
-            if (mrow) s += __half2float(__ldg(mrow + kc)) * 1.4426950408889634f;
-            return s;
-        };
-        // running max / sum of one key block (reads S twice: max, then sum)
-        auto block_stats = [&](int kbase, float& m_run, float& l_run) {
+        // this thread's 64 scores of task t, scaled and masked (log2 domain); frees the buffer
+        auto fetch = [&](float (&s)[64], int kbase, int j) -> float {
+            uint32_t v0[32], v1[32];
+            const uint32_t addr = tmem_base + (t & 1) * BKV + lane_off + hf * 64;
+            tmem_ld32(addr, v0);
+            tmem_ld32(addr + 32, v1);
+            tmem_ld_wait_regs(v0);
+            tmem_ld_wait_regs(v1);
+            tc_fence_before_sync();
+            mbar_arrive(&s_free[t & 1]);
             float mx = NINF;
-#pragma unroll 1
-            for (int c = 0; c < BKV / 32; ++c) {
-                uint32_t v[32];
-                tmem_ld32(tmem_S + lane_off + c * 32, v);
-                tmem_ld_wait();
 #pragma unroll
-                for (int i = 0; i < 32; ++i) mx = fmaxf(mx, score(v[i], kbase + c * 32 + i));
-            }
-            const float m_new = fmaxf(m_run, mx);
-            const float m_use = (m_new == NINF) ? 0.f : m_new;
-            float sum = 0.f;
-#pragma unroll 1
-            for (int c = 0; c < BKV / 32; ++c) {
-                uint32_t v[32];
-                tmem_ld32(tmem_S + lane_off + c * 32, v);
-                tmem_ld_wait();
+            for (int i = 0; i < 64; ++i)
+                s[i] = __uint_as_float(i < 32 ? v0[i & 31] : v1[i & 31]) * a.scale_log2;
+            const bool need_mask = (j * BKV + BKV > kv_len) || (MASK == ET_MASK_ADDITIVE) ||
+                                   (MASK == ET_MASK_CAUSAL && j * BKV + BKV - 1 > q0);
+            if (need_mask) {
 #pragma unroll
-                for (int i = 0; i < 32; ++i) sum += exp2_approx(score(v[i], kbase + c * 32 + i) - m_use);
+                for (int i = 0; i < 64; ++i) {
+                    const int kc = kbase + i;
+                    if (kc >= kv_len || (MASK == ET_MASK_CAUSAL && kc > qrow)) s[i] = NINF;
+                    else if (MASK == ET_MASK_ADDITIVE && mrow)
+                        s[i] += __half2float(__ldcg(reinterpret_cast<const __half*>(mrow + kc))) *
+                                1.4426950408889634f;
+                }
             }
-            l_run = l_run * exp2_approx(m_run - m_use) + sum;
-            m_run = m_new;
+#pragma unroll
+            for (int i = 0; i < 64; ++i) mx = fmaxf(mx, s[i]);
+            return mx;
+        };
+        auto wait_scores = [&]() -> bool {
+            bool good = mbar_wait_bounded(&s_full[t & 1], (t >> 1) & 1, abort_flag);
+            good = __all_sync(0xffffffffu, good);
+            if (good) tc_fence_after_sync();
+            return good;
         };
 
-        for (int h = 0; ok && h < a.nhead; ++h) {
-            float m_run = NINF, l_run = 0.f;
+        // A warp whose wait ran out keeps walking (every later wait is skipped), so that the pair
+        // barriers match.
+        for (int h = h_begin; n_kv > 0 && h < h_end; ++h) {
+            float m_use = 0.f, inv = 0.f;
             if (passes == 2) {
+                // each half keeps a running max and sum of its own keys; the halves meet once
+                float m_run = NINF, l_run = 0.f;
                 for (int j = 0; j < n_kv; ++j) {
-                    ok = mbar_wait_bounded(s_full, t_s & 1, abort_flag);
-                    ok = __all_sync(0xffffffffu, ok);
-                    if (!ok) break;
-                    tc_fence_after_sync();
-                    block_stats(j * BKV, m_run, l_run);
-                    tc_fence_before_sync();
-                    mbar_arrive(s_free);
-                    ++t_s;
+                    ok = ok && wait_scores();
+                    float s[64];
+                    const float mx = fetch(s, j * BKV + hf * 64, j);
+                    const float m_new = fmaxf(m_run, mx);
+                    const float neg = (m_new == NINF) ? 0.f : -m_new;
+                    float sum = 0.f;
+#pragma unroll
+                    for (int i = 0; i < 64; ++i) sum += exp2_approx(s[i] + neg);
+                    l_run = l_run * exp2_approx(m_run + neg) + sum;
+                    m_run = m_new;
+                    ++t;
                 }
-                if (!ok) break;
+                x_a[hf * BQ + r] = m_run;
+                x_b[hf * BQ + r] = l_run;
+                pair_sync();
+                const float m_o = x_a[(hf ^ 1) * BQ + r], l_o = x_b[(hf ^ 1) * BQ + r];
+                const float m_all = fmaxf(m_run, m_o);
+                m_use = (m_all == NINF) ? 0.f : m_all;
+                // (the same order of addition in both halves)
+                const float l0 = (hf == 0 ? l_run : l_o) * exp2_approx((hf == 0 ? m_run : m_o) - m_use);
+                const float l1 = (hf == 0 ? l_o : l_run) * exp2_approx((hf == 0 ? m_o : m_run) - m_use);
+                const float l_all = l0 + l1;
+                inv = l_all > 0.f ? 1.0f / l_all : 0.f;
+                pair_sync();  // the exchange slots are free for the next head
             }
             for (int j = 0; j < n_kv; ++j) {
-                ok = mbar_wait_bounded(s_full, t_s & 1, abort_flag);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
-                tc_fence_after_sync();
-                if (passes == 1) block_stats(j * BKV, m_run, l_run);
-                const float m_use = (m_run == NINF) ? 0.f : m_run;
-                const float inv = l_run > 0.f ? 1.0f / l_run : 0.f;
-                if (t_b > 0) {
+                ok = ok && wait_scores();
+                float s[64];
+                const float mx = fetch(s, j * BKV + hf * 64, j);
+                if (passes == 1) {
+                    x_a[hf * BQ + r] = mx;
+                    pair_sync();
+                    const float m_all = fmaxf(mx, x_a[(hf ^ 1) * BQ + r]);
+                    m_use = (m_all == NINF) ? 0.f : m_all;
+                }
+                float sum = 0.f;
+#pragma unroll
+                for (int i = 0; i < 64; ++i) {
+                    s[i] = exp2_approx(s[i] - m_use);
+                    sum += s[i];
+                }
+                if (passes == 1) {
+                    x_b[hf * BQ + r] = sum;
+                    pair_sync();
+                    const float l_all = x_b[r] + x_b[BQ + r];
+                    inv = l_all > 0.f ? 1.0f / l_all : 0.f;
+                }
+                uint32_t p[32];
+#pragma unroll
+                for (int i = 0; i < 32; ++i) p[i] = pack_half2(s[2 * i] * inv, s[2 * i + 1] * inv);
+                if (ok && t_b > 0) {  // the previous product has read the P tile
                     ok = mbar_wait_bounded(pv_done, (t_b - 1) & 1, abort_flag);
                     ok = __all_sync(0xffffffffu, ok);
-                    if (!ok) break;
                 }
-                const int kbase = j * BKV;
-#pragma unroll 1
-                for (int c = 0; c < BKV / 32; ++c) {
-                    uint32_t v[32];
-                    tmem_ld32(tmem_S + lane_off + c * 32, v);
-                    tmem_ld_wait();
-                    float p[32];
+                uint8_t* prow = sP + hf * ATOM_BYTES + r * 128;
 #pragma unroll
-                    for (int i = 0; i < 32; ++i)
-                        p[i] = exp2_approx(score(v[i], kbase + c * 32 + i) - m_use) * inv;
-                    uint8_t* prow = sP + (c >> 1) * ATOM_BYTES + r * 128;
-#pragma unroll
-                    for (int g = 0; g < 4; ++g) {
-                        uint4 pk;
-                        pk.x = pack_half2(p[g * 8 + 0], p[g * 8 + 1]);
-                        pk.y = pack_half2(p[g * 8 + 2], p[g * 8 + 3]);
-                        pk.z = pack_half2(p[g * 8 + 4], p[g * 8 + 5]);
-                        pk.w = pack_half2(p[g * 8 + 6], p[g * 8 + 7]);
-                        const int chunk = ((c & 1) * 4 + g) ^ (r & 7);
-                        *reinterpret_cast<uint4*>(prow + chunk * 16) = pk;
-                    }
-                }
-                tc_fence_before_sync();
-                mbar_arrive(s_free);
+                for (int g = 0; g < 8; ++g)
+                    *reinterpret_cast<uint4*>(prow + ((g ^ (r & 7)) * 16)) =
+                        make_uint4(p[4 * g], p[4 * g + 1], p[4 * g + 2], p[4 * g + 3]);
                 fence_proxy_async_smem();
                 mbar_arrive(p_full);
-                ++t_s;
+                ++t;
                 ++t_b;
             }
         }
-        if (!ok) report_error(a.err_word, abort_flag, DEV_TIMEOUT_VO_SOFTMAX);
-
         if (ok && t_b > 0) {
             ok = mbar_wait_bounded(pv_done, (t_b - 1) & 1, abort_flag);
-            if (!ok) report_error(a.err_word, abort_flag, DEV_TIMEOUT_VO_SOFTMAX);
             ok = __all_sync(0xffffffffu, ok);
         }
-        if (ok) {
-            tc_fence_after_sync();
-            __half* orow = a.out + (static_cast<size_t>(b) * a.seq + (qrow < a.seq ? qrow : 0)) * a.emdim + e0;
-            for (int c = 0; c < (n_c >> 4); ++c) {
-                uint32_t o[16];
-                if (t_b > 0) {
-                    tmem_ld16(tmem_O + lane_off + c * 16, o);
-                    tmem_ld_wait();
-                } else {
+        if (!ok) report_error(a.err_word, abort_flag, DEV_TIMEOUT_VO_SOFTMAX);
+        tc_fence_after_sync();
+    }
+
+    // ---------------- the heads' partial sums meet, rows dealt to the ranks ----------------
+    // Every product of every CTA is complete, so the operand stages may be overwritten.  (A CTA
+    // whose wait ran out takes the same barriers.)
+    __syncwarp();
+    if (csize > 1) cluster_sync_all(); else __syncthreads();
+    const int rows_per = (BQ + csize - 1) / csize;
+    constexpr int pitch = vo_pitch(NC);
+    if (warp >= 3 && !*abort_flag) {
+        const int qd = warp & 3;
+        const int hf = (warp - 3) >> 2;
+        const int r = qd * 32 + lane;
+        const uint32_t lane_off = static_cast<uint32_t>(qd * 32) << 16;
+        const int owner = r / rows_per;
+        const uint32_t local = smem_u32(smem + (rank * rows_per + (r - owner * rows_per)) * pitch);
+        const uint32_t dst = csize > 1 ? map_to_cta(local, owner) : local;
+        for (int c = hf; c < (n_c >> 4); c += 2) {
+            uint32_t o[16];
+            if (n_task > 0) {
+                tmem_ld16(tmem_O + lane_off + c * 16, o);
+                tmem_ld_wait();
+            } else {
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) o[i] = 0u;
-                }
-                if (qrow < a.seq) {
-                    float f[16];
+                for (int i = 0; i < 16; ++i) o[i] = 0u;
+            }
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) f[i] = __uint_as_float(o[i]);
-                    if (a.bias_o != nullptr) {
+            for (int g = 0; g < 4; ++g)
+                st_cluster_v4(dst + c * 64 + g * 16, o[4 * g], o[4 * g + 1], o[4 * g + 2], o[4 * g + 3]);
+        }
+    }
+    __syncwarp();
+    if (csize > 1) cluster_sync_all(); else __syncthreads();
+    if (!*abort_flag) {
+        const int r0 = rank * rows_per;
+        int nrow = BQ - r0 < rows_per ? BQ - r0 : rows_per;
+        nrow = a.seq - q0 - r0 < nrow ? a.seq - q0 - r0 : nrow;
+        const int pieces = n_c >> 3;
+        for (int i = threadIdx.x; i < nrow * pieces; i += VO_THREADS) {
+            const int rl = i / pieces, c = (i - rl * pieces) * 8;
+            float f[8];
 #pragma unroll
-                        for (int g = 0; g < 2; ++g) {
-                            const uint4 bq =
-                                __ldg(reinterpret_cast<const uint4*>(a.bias_o + e0 + c * 16 + g * 8));
-                            const __half2* bh = reinterpret_cast<const __half2*>(&bq);
+            for (int k = 0; k < 8; ++k) f[k] = 0.f;
+            for (int g = 0; g < csize; ++g) {
+                const float4* src =
+                    reinterpret_cast<const float4*>(smem + (g * rows_per + rl) * pitch + c * 4);
+                const float4 u = src[0], w = src[1];
+                f[0] += u.x; f[1] += u.y; f[2] += u.z; f[3] += u.w;
+                f[4] += w.x; f[5] += w.y; f[6] += w.z; f[7] += w.w;
+            }
+            if (a.bias_o != nullptr) {
+                const uint4 bq = __ldg(reinterpret_cast<const uint4*>(a.bias_o + e0 + c));
+                const __half2* bh = reinterpret_cast<const __half2*>(&bq);
 #pragma unroll
-                            for (int i = 0; i < 4; ++i) {
-                                const float2 bf = __half22float2(bh[i]);
-                                f[g * 8 + 2 * i] += bf.x;
-                                f[g * 8 + 2 * i + 1] += bf.y;
-                            }
-                        }
-                    }
-                    uint4 w0, w1;
-                    w0.x = pack_half2(f[0], f[1]);
-                    w0.y = pack_half2(f[2], f[3]);
-                    w0.z = pack_half2(f[4], f[5]);
-                    w0.w = pack_half2(f[6], f[7]);
-                    w1.x = pack_half2(f[8], f[9]);
-                    w1.y = pack_half2(f[10], f[11]);
-                    w1.z = pack_half2(f[12], f[13]);
-                    w1.w = pack_half2(f[14], f[15]);
-                    *reinterpret_cast<uint4*>(orow + c * 16) = w0;
-                    *reinterpret_cast<uint4*>(orow + c * 16 + 8) = w1;
+                for (int k = 0; k < 4; ++k) {
+                    const float2 bf = __half22float2(bh[k]);
+                    f[2 * k] += bf.x;
+                    f[2 * k + 1] += bf.y;
                 }
             }
+            uint4 w;
+            w.x = pack_half2(f[0], f[1]);
+            w.y = pack_half2(f[2], f[3]);
+            w.z = pack_half2(f[4], f[5]);
+            w.w = pack_half2(f[6], f[7]);
+            *reinterpret_cast<uint4*>(a.out + (static_cast<size_t>(b) * a.seq + q0 + r0 + rl) * a.emdim +
+                                      e0 + c) = w;
         }
     }
 
     tc_fence_before_sync();
     __syncthreads();
-    if (warp == 1) tmem_dealloc(tmem_base, vo_tmem_cols(NC));
+    if (warp == 1) tmem_dealloc(tmem_base, VO_TMEM_COLS);
 }
 
 }  // namespace
@@ -418,8 +543,8 @@ int et_fused_vo_attention_fwd(const et_half* Q, const et_half* K, const et_half*
     if (!err) return ET_ERR_NO_DEVICE;
 
     CUtensorMap tmQ, tmK, tmVO;
-    const uint32_t box[3] = {64, 128, 1};
-    auto make = [&](CUtensorMap* m, const void* p, int ld, int width, int groups) {
+    auto make = [&](CUtensorMap* m, const void* p, int ld, int width, int groups, uint32_t rows) {
+        const uint32_t box[3] = {64, rows, 1};
         const uint64_t dims[3] = {static_cast<uint64_t>(width), static_cast<uint64_t>(seq),
                                   static_cast<uint64_t>(groups)};
         const uint64_t strides[2] = {static_cast<uint64_t>(ld) * 2,
@@ -427,9 +552,9 @@ int et_fused_vo_attention_fwd(const et_half* Q, const et_half* K, const et_half*
         return make_tensor_map_f16(m, p, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
     };
     int st;
-    if ((st = make(&tmQ, Q, ldq, nhead * dh_qk, batch)) != ET_OK) return st;
-    if ((st = make(&tmK, K, ldk, nhead * dh_qk, batch)) != ET_OK) return st;
-    if ((st = make(&tmVO, VO, emdim, emdim, batch * nhead)) != ET_OK) return st;
+    if ((st = make(&tmQ, Q, ldq, nhead * dh_qk, batch, BQ)) != ET_OK) return st;
+    if ((st = make(&tmK, K, ldk, nhead * dh_qk, batch, BKV)) != ET_OK) return st;
+    if ((st = make(&tmVO, VO, emdim, emdim, batch * nhead, VO_KEYS)) != ET_OK) return st;
 
     VoArgs a;
     a.out = reinterpret_cast<__half*>(out);
@@ -441,38 +566,63 @@ int et_fused_vo_attention_fwd(const et_half* Q, const et_half* K, const et_half*
     a.nhead = nhead;
     a.dh_qk = dh_qk;
     a.emdim = emdim;
-    a.mask_kind = mask_kind;
     a.scale_log2 = scale * 1.4426950408889634f;
     a.err_word = err;
-    // Measured on B200 (12 heads, 768 features; 256 / 128 / 64 features per CTA): 16 x 128 tokens
-    // 188 / 195 / 202 us, 64 x 128 376 / 385 / 603, 4 x 512 762 / 794 / 829, 1 x 4096 6.1 / 6.6 /
-    // 12.5 ms, and 181-186 us for a single 128-token sequence whatever the width: a CTA's time is
-    // set by its serial walk over the heads (about 15 us per head and key block with one set of
-    // buffers), not by how many CTAs there are, so the widest chunk runs unless the test hook
-    // asks for another.
+    // Heads are dealt to as many CTAs per item (up to 8, a portable cluster) as keep the launch
+    // within one CTA per SM: a CTA's time is its serial walk over its heads.  The count is taken
+    // for 256-feature items whatever the chunk width, so that every width adds the heads' partial
+    // sums in the same order.
     int nc = 256;
     if (g_vo_chunk == 64 || g_vo_chunk == 128) nc = g_vo_chunk;
-    const int nqa = (dh_qk + 63) / 64;
+    const int sms = sm_count() > 0 ? sm_count() : 148;
+    const long qblocks = (seq + BQ - 1) / BQ;
+    const long items = qblocks * ((emdim + 255) / 256) * batch;
+    long csize = sms / items;
+    csize = csize > VO_MAX_CLUSTER ? VO_MAX_CLUSTER : csize;
+    csize = csize > nhead ? nhead : csize;
+    csize = csize < 1 ? 1 : csize;
     int dev = 0;
     cudaGetDevice(&dev);
     auto go = [&](auto kern, int slot, int width) -> int {
-        const int smem_bytes = (2 * nqa + width / 64 + 2) * ATOM_BYTES + 256 + 1024;
-        static std::atomic<bool> attr_set[3][64] = {};
+        const int smem_bytes = vo_smem_bytes(width);
+        static std::atomic<bool> attr_set[12][64] = {};
         if (dev >= 0 && dev < 64 && !attr_set[slot][dev]) {
-            if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (2 * 2 + width / 64 + 2) * ATOM_BYTES + 256 + 1024) != cudaSuccess)
+            if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes) !=
+                cudaSuccess)
                 return ET_ERR_CUDA;
             attr_set[slot][dev] = true;
         }
-        dim3 grid((seq + BQ - 1) / BQ, (emdim + width - 1) / width, batch);
-        return launch_kernel(kern, grid, dim3(VO_THREADS), smem_bytes,
-                             static_cast<cudaStream_t>(stream), tmQ, tmK, tmVO, a) == cudaSuccess
-                   ? ET_OK
-                   : ET_ERR_CUDA;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(static_cast<unsigned>(csize * qblocks),
+                           static_cast<unsigned>((emdim + width - 1) / width), static_cast<unsigned>(batch));
+        cfg.blockDim = dim3(VO_THREADS);
+        cfg.dynamicSmemBytes = static_cast<size_t>(smem_bytes);
+        cfg.stream = static_cast<cudaStream_t>(stream);
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = static_cast<unsigned>(csize);
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = pdl_enabled() ? 2 : 1;
+        count_launch();
+        return cudaLaunchKernelEx(&cfg, kern, tmQ, tmK, tmVO, a) == cudaSuccess ? ET_OK : ET_ERR_CUDA;
     };
-    if (nc == 64) return go(attention_vo_kernel<64>, 0, 64);
-    if (nc == 128) return go(attention_vo_kernel<128>, 1, 128);
-    return go(attention_vo_kernel<256>, 2, 256);
+    auto by_mask = [&](auto width) -> int {
+        constexpr int W = decltype(width)::value;
+        constexpr int base = W == 256 ? 0 : (W == 128 ? 4 : 8);
+        switch (mask_kind) {
+            case ET_MASK_CAUSAL: return go(attention_vo_kernel<W, ET_MASK_CAUSAL>, base + 1, W);
+            case ET_MASK_PADDING: return go(attention_vo_kernel<W, ET_MASK_PADDING>, base + 2, W);
+            case ET_MASK_ADDITIVE: return go(attention_vo_kernel<W, ET_MASK_ADDITIVE>, base + 3, W);
+            default: return go(attention_vo_kernel<W, ET_MASK_NONE>, base, W);
+        }
+    };
+    if (nc == 64) return by_mask(std::integral_constant<int, 64>{});
+    if (nc == 128) return by_mask(std::integral_constant<int, 128>{});
+    return by_mask(std::integral_constant<int, 256>{});
 }
 
 #ifdef ET_TEST_HOOKS

@@ -73,9 +73,11 @@ struct TileCoord {
 // B_MN == true : W is [groups][K, N] with N contiguous; its tiles are consumed in place
 //                as MN-major operands (64-column atoms of 64 K-rows, 8 KB each).
 // EPI: 0 = every output mode and activation chosen at run time (index-list, grouped and
-// partial-sum epilogues); 1 + act = the fp16 tile store with that activation compiled in.  The
-// specialised form matters: with all variants inlined behind run-time branches the same
-// staging code ran three times slower.
+// partial-sum epilogues); 1 + act = the fp16 tile store with that activation compiled in;
+// EPI_GROUPED = the grouped rows of the V.O projection through the staging tile and 16-byte row
+// stores.  The specialised forms matter: with all variants inlined behind run-time branches the
+// same staging code ran three times slower.
+constexpr int EPI_GROUPED = 4;
 template <int BN, int STAGES, bool PERSIST, bool B_MN, int EPI>
 __global__ void __launch_bounds__(GEMM_THREADS, (GemmCfg<BN, STAGES, PERSIST>::MIN_CTAS))
 gemm_f16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
@@ -322,9 +324,37 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             }
 
             auto finish_chunk = [&](int ch, const uint32_t (&r)[32]) {
+                if (EPI == EPI_GROUPED) {
+                    // Row m of group z lands between the other groups' rows of its sequence, so the
+                    // 32 staged rows are written one by one: eight lanes per 128-byte row piece.
+                    // (Element stores straight from the accumulator's layout, one row per lane,
+                    // cost 32 sectors per instruction: 12 x 2048 x 768 x 768 took 190 us.)
+                    uint8_t* tile = sStage + (q * (BN / 64) + (ch >> 1)) * 4096;
+                    stage_f16_chunk<ET_ACT_NONE>(r, tb + ch * 32, tile + lane * 128, ch & 1, lane);
+                    if ((ch & 1) || c.n0 + ch * 32 + 32 >= N) {
+                        __syncwarp();
+                        const int piece = lane & 7, n = c.n0 + (ch >> 1) * 64 + piece * 8;
+                        __half* Y = static_cast<__half*>(g.Y);
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            const int rr = i * 4 + (lane >> 3), m = c.m0 + q * 32 + rr;
+                            if (m < M && n < N) {
+                                const int sq = m / g.grp_rows;
+                                const size_t out_row = static_cast<size_t>(sq) * g.grp_stride +
+                                                       static_cast<size_t>(grp) * g.grp_rows +
+                                                       (m - sq * g.grp_rows);
+                                *reinterpret_cast<uint4*>(Y + out_row * g.ldy + n) =
+                                    *reinterpret_cast<const uint4*>(tile + rr * 128 +
+                                                                    ((piece ^ (rr & 7)) * 16));
+                            }
+                        }
+                        __syncwarp();
+                    }
+                    return;
+                }
                 if (EPI != 0) {
                     uint8_t* tile = sStage + (q * (BN / 64) + (ch >> 1)) * 4096;
-                    stage_f16_chunk<EPI - 1>(r, tb + ch * 32, tile + lane * 128, ch & 1, lane);
+                    stage_f16_chunk<EPI == EPI_GROUPED ? ET_ACT_NONE : EPI - 1>(r, tb + ch * 32, tile + lane * 128, ch & 1, lane);
                     if ((ch & 1) || c.n0 + ch * 32 + 32 >= N) {  // the 64-column group is complete
                         fence_proxy_async_smem();
                         __syncwarp();
@@ -362,12 +392,9 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                     if (lane == 0 && c.m0 + q * 32 < M)
                         tma_store_3d(&tmY, tile, c.n0 + ch * 32, c.m0 + q * 32, c.z);
                 } else if (row < M) {
-                    // index-list / grouped-row epilogues: direct stores (small problems only)
+                    // index-list epilogue: direct stores (small problems only)
                     __half* Y = static_cast<__half*>(g.Y);
-                    size_t out_row = static_cast<size_t>(row);
-                    if (g.grp_rows > 0)
-                        out_row = static_cast<size_t>(row / g.grp_rows) * g.grp_stride +
-                                  static_cast<size_t>(grp) * g.grp_rows + row % g.grp_rows;
+                    const size_t out_row = static_cast<size_t>(row);
 #pragma unroll
                     for (int j = 0; j < 32; ++j) {
                         const int n = c.n0 + ch * 32 + j;
@@ -650,7 +677,8 @@ int launch_cfg(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap
             return launch_cfg_epi<BN, STAGES, PERSIST, false, 1 + ET_ACT_RELU>(tmA, tmB, tmY, args, zdim, stream);
         return launch_cfg_epi<BN, STAGES, PERSIST, false, 1 + ET_ACT_NONE>(tmA, tmB, tmY, args, zdim, stream);
     }
-    return launch_cfg_epi<BN, STAGES, PERSIST, B_MN, 0>(tmA, tmB, tmY, args, zdim, stream);
+    return launch_cfg_epi<BN, STAGES, PERSIST, B_MN, B_MN ? EPI_GROUPED : 0>(tmA, tmB, tmY, args, zdim,
+                                                                            stream);
 }
 
 int g_force_bn = 0;       // test hook: 0 = automatic, else 64 / 128 / 192 / 256 / 384
@@ -941,8 +969,7 @@ int launch_gemm_f16_grouped_kn(const __half* X, int ldx, const __half* W, const 
     if (!device_error_word()) return ET_ERR_NO_DEVICE;
     TilePlan plan = pick_plan(M, N, K, groups);
     if (plan.bn == 384) plan = TilePlan{128, plan_tiles(M, N, 128) * groups > sm_count()};
-    if (plan.bn == 256 || plan.bn == 192) plan.bn = 128;
-    const int bn = plan.bn;
+    if (plan.bn == 192) plan.bn = 256;  // (no 192-wide MN-major form)
     CUtensorMap tmA, tmB;
     int st;
     if ((st = encode_operand(&tmA, X, ldx, M, K, BM)) != ET_OK) return st;
@@ -959,7 +986,6 @@ int launch_gemm_f16_grouped_kn(const __half* X, int ldx, const __half* W, const 
     args.out_mode = OUT_GROUPED;
     args.grp_rows = grp_rows;
     args.grp_stride = groups * grp_rows;
-    (void)bn;
     return dispatch<true>(plan, tmA, tmB, tmA, args, groups, stream);
 }
 
