@@ -424,6 +424,27 @@ __device__ __forceinline__ void mma_f16_ss(uint32_t d_tmem, uint64_t a_desc, uin
         : "memory");
 }
 
+// The same product for two K-major operands in 128-byte-swizzled tiles, the descriptors given by
+// their low words (desc_lo of the address, + 2 per 16 columns): everything else in them is fixed.
+__device__ __forceinline__ uint32_t desc_lo(uint32_t smem_addr) {
+    return ((smem_addr & 0x3FFFFu) >> 4) | (1u << 16);  // leading byte offset 16
+}
+constexpr uint32_t DESC_HI_K128 = (1024u >> 4) | (1u << 14) | (2u << 29);  // stride 1024, 128 B swizzle
+__device__ __forceinline__ void mma_f16_ss_k128(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo,
+                                                uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        ".reg .b64 da, db;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "mov.b64 da, {%1, %5};\n\t"
+        "mov.b64 db, {%2, %5};\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n\t"
+        "}\n"
+        ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "n"(DESC_HI_K128)
+        : "memory");
+}
+
 // Arrives on the mbarrier once every tcgen05.mma issued so far by this thread is done.
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::

@@ -211,6 +211,8 @@ int launch_linear_tile_packed(const int* row_ptr, const uint32_t* pk_mask, const
     if (nnz_tiles > 0 && tile_packed_mode() == 1)
         return launch_linear_tile_persist(row_ptr, pk_mask, pk_off, pk_tiles, nnz_tiles, bias, X, Y, T, in,
                                           out, act, stream);
+    if (nnz_tiles > 0 && tile_packed_mode() == 2 && in % 16 == 0 && out % 16 == 0)
+        return launch_linear_expand_packed(pk_mask, pk_off, pk_tiles, bias, X, Y, T, in, out, act, stream);
     return launch_tile_common(true, row_ptr, nullptr, pk_mask, pk_off, pk_tiles, nnz_tiles, bias, X, Y,
                               T, in, out, act, stream);
 }

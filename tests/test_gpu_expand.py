@@ -1,0 +1,102 @@
+"""GPU parity of the Linear layers whose weights are expanded to operand tiles in shared memory
+(1x16 vectors, CSR, packed tiles) at the edges of their tiling: partial token blocks, several
+token blocks per CTA, partial feature panels of every width, K not a multiple of a block, weight
+buffers that wrap, empty and full weights; CSR rows in any order and with repeated columns.
+
+Tolerance: both sides accumulate fp16 products in fp32, so they differ by the rounding of the fp16
+output, at most 2^-11 of the largest |y|, plus fp32 summation order (K * 2^-24 of sum |w x|, far
+below it).  GELU adds the 5e-4 absolute error of tanh.approx."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [
+    # T, in, out
+    (1, 16, 16), (128, 768, 768), (129, 80, 144), (300, 1024, 48), (700, 1040, 3088), (2048, 256, 2304),
+    (4100, 192, 1008), (64, 3072, 768),
+]
+
+
+def _dev(a, cuda):
+    import torch
+    return torch.from_numpy(np.ascontiguousarray(a)).to(cuda)
+
+
+def _check(y, ref, what):
+    y = y.float().cpu().numpy()
+    tol = 2.0 ** -11 * np.abs(ref).max() + 6e-4
+    assert np.isfinite(y).all() and np.abs(y - ref).max() <= tol, f"{what}: {np.abs(y - ref).max()} > {tol}"
+
+
+def _case(et, seed, T, inn, out):
+    return (et.synth.normal_fast(seed, 1, (T, inn), 1.0), et.synth.normal_fast(seed, 2, (out, inn), 0.05),
+            et.synth.normal_fast(seed, 3, (out,), 0.1))
+
+
+@pytest.mark.parametrize("sparsity", [0.0, 0.9, 1.0])
+@pytest.mark.parametrize("T,inn,out", SHAPES)
+def test_1x16(et, orc, cuda, T, inn, out, sparsity):
+    x, w, b = _case(et, 71, T, inn, out)
+    w = et.synth.prune_1x16(w, 71, 6, sparsity)
+    ti, ri, data = et.synth.dense_to_1x16(w)
+    n = len(ri)
+    y = et.linear_1x16(_dev(x, cuda), _dev(ti, cuda), _dev(ri, cuda) if n else None,
+                       _dev(data, cuda) if n else None, out, _dev(b, cuda), 2)
+    assert et.device_error() == 0
+    _check(y, orc.linear_dense(x, w, b, 2), f"1x16 {T}x{inn}x{out} s={sparsity}")
+
+
+@pytest.mark.parametrize("sparsity", [0.5, 0.97])
+@pytest.mark.parametrize("T,inn,out", SHAPES + [(130, 8192, 40), (77, 1000, 203), (260, 24, 5)])
+def test_csr(et, orc, cuda, T, inn, out, sparsity):
+    x, w, b = _case(et, 72, T, inn, out)
+    w = w * (et.synth.uniform(72, 7, out * inn).reshape(out, inn) >= sparsity)
+    ip, ix, data = et.synth.dense_to_csr(w)
+    n = len(ix)
+    y = et.linear_csr(_dev(x, cuda), _dev(ip, cuda), _dev(ix, cuda) if n else None,
+                      _dev(data, cuda) if n else None, out, _dev(b, cuda), 1)
+    assert et.device_error() == 0
+    _check(y, orc.linear_dense(x, w, b, 1), f"csr {T}x{inn}x{out} s={sparsity}")
+
+
+@pytest.mark.parametrize("inn", [256, 3072])
+def test_csr_rows_in_any_order_and_repeated_columns(et, orc, cuda, inn):
+    T, out = 200, 100
+    x, w, b = _case(et, 73, T, inn, out)
+    rng = np.random.default_rng(5)
+    ip, ix, data = [0], [], []
+    for r in range(out):
+        cols = rng.permutation(inn)[:20]
+        if r % 7 == 3:
+            cols[5] = cols[11]  # one column twice: its values add up
+        ix += list(cols)
+        data += list(w[r, rng.permutation(inn)[:20]])
+        ip.append(len(ix))
+    ip, ix, data = np.array(ip, np.int32), np.array(ix, np.int32), np.array(data, np.float16)
+    y = et.linear_csr(_dev(x, cuda), _dev(ip, cuda), _dev(ix, cuda), _dev(data, cuda), out, _dev(b, cuda), 0)
+    assert et.device_error() == 0
+    _check(y, orc.linear_csr(x, ip, ix, data, out, b, 0), f"unordered csr, in {inn}")
+
+
+@pytest.mark.parametrize("sparsity", [0.0, 0.8, 0.95])
+@pytest.mark.parametrize("T,inn,out", SHAPES)
+def test_packed_tiles(et, orc, cuda, T, inn, out, sparsity):
+    import ctypes
+    import torch
+    x, w, b = _case(et, 74, T, inn, out)
+    w = et.synth.prune_tiles(w, 74, 4, sparsity)
+    rp, ro, tiles = et.synth.dense_to_tile(w)
+    pk = et.PackedTiles(rp, ro, tiles, inn, out, cuda)
+    L = et.lib()
+    ys = []
+    for mode in (2, 0):  # expanded tiles; one tensor-core product per stored tile
+        L.et_debug_set_tile_persist(ctypes.c_int(mode))
+        try:
+            ys.append(et.linear_tile_packed(_dev(x, cuda), pk, _dev(b, cuda), 2))
+            assert et.device_error() == 0
+        finally:
+            L.et_debug_set_tile_persist(ctypes.c_int(-1))
+    _check(ys[0], orc.linear_dense(x, w, b, 2), f"packed {T}x{inn}x{out} s={sparsity}")
+    # the products of absent tiles add exact zeros: the same bits
+    assert torch.equal(ys[0], ys[1])
