@@ -139,7 +139,7 @@ __device__ __forceinline__ void attention_cta(const CUtensorMap& tmQ, const CUte
     volatile int* abort_flag = FUSED ? abort_in : reinterpret_cast<volatile int*>(tmem_slot + 1);
     float* s_xmax = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + 256);
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = uniform_warp_id();
     const int lane = threadIdx.x & 31;
 
     // V window of this head: feature offset v_x0 (a multiple of 8 so the TMA start is 16-byte
@@ -240,14 +240,19 @@ __device__ __forceinline__ void attention_cta(const CUtensorMap& tmQ, const CUte
             }
         }
     } else if (warp == 1) {
-        // ---------------- MMA issuer ----------------
-        if (n_kv > 0 && elect_one()) {
+        // ---------------- MMA issuer (warp-uniform, one elected lane issues) ----------------
+        if (n_kv > 0) {
+            const bool leader = elect_one();
             const uint32_t idesc_s = make_idesc_f16(BQ, BKV, 0, 0);
             const uint32_t idesc_o = make_idesc_f16(BQ, v_n, 0, 1);  // V is MN-major
-            const uint32_t q_addr = smem_u32(sQ), k_addr = smem_u32(sK), v_addr = smem_u32(sV),
-                           p_addr = smem_u32(sP);
+            const uint32_t q_lo = desc_lo(smem_u32(sQ)), k_lo = desc_lo(smem_u32(sK)),
+                           p_lo = desc_lo(smem_u32(sP));
+            // V tile: 16 keys = two groups of 8 rows of 128 bytes (SBO = 1024); a second
+            // 64-feature atom sits ATOM_BYTES further (LBO).
+            const uint32_t v_lo =
+                ((smem_u32(sV) & 0x3FFFFu) >> 4) | (static_cast<uint32_t>(ATOM_BYTES >> 4) << 16);
+            const int ksteps = a.dh_qk >> 4;
             bool ok = mbar_wait_bounded(q_full, 0, abort_flag);
-            if (!ok) report_error(a.err_word, abort_flag, DEV_TIMEOUT_ATTN_MMA);
             // S_j = Q.K_j^T; the score block is free as soon as the softmax warps hold it in
             // registers, so S_{j+1} is issued BEFORE P_j.V_j and runs under softmax(j).
             auto issue_s = [&](int j) -> bool {
@@ -256,52 +261,47 @@ __device__ __forceinline__ void attention_cta(const CUtensorMap& tmQ, const CUte
                       mbar_wait_bounded(s_free, ph ^ 1, abort_flag)))
                     return false;
                 tc_fence_after_sync();
-                const int ksteps = a.dh_qk >> 4;
-                for (int kk = 0; kk < ksteps; ++kk) {
-                    const uint32_t off = (kk >> 2) * ATOM_BYTES + (kk & 3) * 32;
-                    mma_f16_ss(tmem_S, make_smem_desc(q_addr + off, 16, 1024, SWZ_128B),
-                               make_smem_desc(k_addr + off, 16, 1024, SWZ_128B), idesc_s,
-                               kk != 0 ? 1u : 0u);
+                if (leader) {
+                    for (int kk = 0; kk < ksteps; ++kk) {
+                        const uint32_t off = (kk >> 2) * (ATOM_BYTES >> 4) + (kk & 3) * 2;
+                        mma_f16_ss_k128(tmem_S, q_lo + off, k_lo + off, idesc_s, kk != 0 ? 1u : 0u);
+                    }
+                    mma_commit(s_full);
+                    mma_commit(k_empty);
                 }
-                mma_commit(s_full);
-                mma_commit(k_empty);
+                __syncwarp();
                 return true;
             };
             if (ok) {
                 ok = issue_s(0);
-                if (!ok) report_error(a.err_word, abort_flag, DEV_TIMEOUT_ATTN_MMA);
-                ET_TL(3);
+                if (leader) ET_TL(3);
             }
             for (int j = 0; ok && j < n_kv; ++j) {
                 const uint32_t ph = j & 1;
                 if (j + 1 < n_kv) ok = issue_s(j + 1);
                 ok = ok && mbar_wait_bounded(p_full, ph, abort_flag) &&
                      mbar_wait_bounded(v_full, ph, abort_flag);
-                if (!ok) {
-                    report_error(a.err_word, abort_flag, DEV_TIMEOUT_ATTN_MMA);
-                    break;
-                }
+                if (!ok) break;
                 tc_fence_after_sync();
+                if (leader) {
 #pragma unroll
-                for (int kk = 0; kk < BKV / 16; ++kk) {
-                    const uint32_t p_off = (kk >> 2) * ATOM_BYTES + (kk & 3) * 32;
-                    // V tile: 16 keys = two groups of 8 rows of 128 bytes (SBO = 1024); a second
-                    // 64-feature atom sits ATOM_BYTES further (LBO).
-                    mma_f16_ss(tmem_O, make_smem_desc(p_addr + p_off, 16, 1024, SWZ_128B),
-                               make_smem_desc(v_addr + kk * 2048, ATOM_BYTES, 1024, SWZ_128B),
-                               idesc_o, (j | kk) != 0 ? 1u : 0u);
+                    for (int kk = 0; kk < BKV / 16; ++kk)
+                        mma_f16_ss_k128(tmem_O, p_lo + (kk >> 2) * (ATOM_BYTES >> 4) + (kk & 3) * 2,
+                                        v_lo + kk * (2048 >> 4), idesc_o, (j | kk) != 0 ? 1u : 0u);
+                    mma_commit(o_full);
+                    mma_commit(v_empty);
+                    if (j == 0) ET_TL(7);
                 }
-                mma_commit(o_full);
-                mma_commit(v_empty);
-                if (j == 0) ET_TL(7);
+                __syncwarp();
             }
             if (FUSED && ok) {
                 // the barriers are invalidated after this piece of work: every arrival a commit
                 // has scheduled must have happened by then
                 ok = mbar_wait_bounded(k_empty, (n_kv - 1) & 1, abort_flag) &&
                      mbar_wait_bounded(v_empty, (n_kv - 1) & 1, abort_flag);
-                if (!ok) report_error(a.err_word, abort_flag, DEV_TIMEOUT_ATTN_MMA);
             }
+            if (!ok && leader) report_error(a.err_word, abort_flag, DEV_TIMEOUT_ATTN_MMA);
+            __syncwarp();
         }
     } else {
         // ---------------- softmax / output warps ----------------

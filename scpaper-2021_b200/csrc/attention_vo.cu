@@ -110,7 +110,7 @@ attention_vo_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     float* s_x = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + 256);  // [2][2][128]
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = uniform_warp_id();
     const int lane = threadIdx.x & 31;
     const int csize = static_cast<int>(vo_cluster_size());
     const int rank = static_cast<int>(cluster_ctarank());
@@ -223,57 +223,70 @@ attention_vo_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                         if (mbar_try_wait(&vo_full[k % VO_STAGES], (k / VO_STAGES) & 1)) break;
         }
     } else if (warp == 1) {
-        // ---------------- MMA issuer ----------------
-        if (n_task > 0 && elect_one()) {
+        // ---------------- MMA issuer (warp-uniform, one elected lane issues) ----------------
+        if (n_task > 0) {
+            const bool leader = elect_one();
             const uint32_t idesc_s = make_idesc_f16(BQ, BKV, 0, 0);
             const uint32_t idesc_o = make_idesc_f16(BQ, n_c, 0, 1);  // VO is MN-major
-            const uint32_t qk_addr = smem_u32(sQK), vo_addr = smem_u32(sVO), p_addr = smem_u32(sP);
+            const uint32_t qk_lo = desc_lo(smem_u32(sQK)), p_lo = desc_lo(smem_u32(sP));
+            const uint32_t vo_lo =
+                ((smem_u32(sVO) & 0x3FFFFu) >> 4) | (static_cast<uint32_t>(VO_ATOM >> 4) << 16);
+            const int ksteps = a.dh_qk >> 4;
             auto issue_s = [&](int t) -> bool {
-                const int s = t % qk_stages;
-                if (!mbar_wait_bounded(&qk_full[s], (t / qk_stages) & 1, abort_flag) ||
+                const int s = t & (qk_stages - 1);
+                if (!mbar_wait_bounded(&qk_full[s], (qk_stages == 2 ? t >> 1 : t) & 1, abort_flag) ||
                     !mbar_wait_bounded(&s_free[t & 1], ((t >> 1) & 1) ^ 1, abort_flag))
                     return false;
                 tc_fence_after_sync();
-                const uint32_t q_addr = qk_addr + s * qk_stage_bytes;
-                const uint32_t k_addr = q_addr + nqa * ATOM_BYTES;
-                for (int kk = 0; kk < (a.dh_qk >> 4); ++kk) {
-                    const uint32_t off = (kk >> 2) * ATOM_BYTES + (kk & 3) * 32;
-                    mma_f16_ss(tmem_base + (t & 1) * BKV, make_smem_desc(q_addr + off, 16, 1024, SWZ_128B),
-                               make_smem_desc(k_addr + off, 16, 1024, SWZ_128B), idesc_s,
-                               kk != 0 ? 1u : 0u);
+                const uint32_t q_lo = qk_lo + s * (qk_stage_bytes >> 4);
+                const uint32_t k_lo = q_lo + nqa * (ATOM_BYTES >> 4);
+                if (leader) {
+                    for (int kk = 0; kk < ksteps; ++kk) {
+                        const uint32_t off = (kk >> 2) * (ATOM_BYTES >> 4) + (kk & 3) * 2;
+                        mma_f16_ss_k128(tmem_base + (t & 1) * BKV, q_lo + off, k_lo + off, idesc_s,
+                                        kk != 0 ? 1u : 0u);
+                    }
+                    mma_commit(&s_full[t & 1]);
+                    mma_commit(&qk_empty[s]);
                 }
-                mma_commit(&s_full[t & 1]);
-                mma_commit(&qk_empty[s]);
+                __syncwarp();
                 return true;
             };
             bool ok = issue_s(0);
             int in_head = 0, t_b = 0, v = 0;
+            uint32_t vph = 0;
             for (int t = 0; ok && t < n_task; ++t) {
                 if (t + 1 < n_task) ok = issue_s(t + 1);
                 if (!ok) break;
                 if (in_head >= per_head - n_kv) {
                     ok = mbar_wait_bounded(p_full, t_b & 1, abort_flag);
-                    for (int half = 0; ok && half < 2; ++half, ++v) {
-                        const int s = v % VO_STAGES;
-                        ok = mbar_wait_bounded(&vo_full[s], (v / VO_STAGES) & 1, abort_flag);
+                    for (int half = 0; ok && half < 2; ++half) {
+                        ok = mbar_wait_bounded(&vo_full[v], vph, abort_flag);
                         if (!ok) break;
                         tc_fence_after_sync();
-                        const uint32_t vb = vo_addr + s * vo_stage_bytes(NC);
+                        if (leader) {
 #pragma unroll
-                        for (int kk = 0; kk < VO_KEYS / 16; ++kk)
-                            mma_f16_ss(tmem_O,
-                                       make_smem_desc(p_addr + half * ATOM_BYTES + kk * 32, 16, 1024, SWZ_128B),
-                                       make_smem_desc(vb + kk * 2048, VO_ATOM, 1024, SWZ_128B), idesc_o,
-                                       (t_b | half | kk) != 0 ? 1u : 0u);
-                        mma_commit(&vo_empty[s]);
+                            for (int kk = 0; kk < VO_KEYS / 16; ++kk)
+                                mma_f16_ss_k128(tmem_O, p_lo + half * (ATOM_BYTES >> 4) + kk * 2,
+                                                vo_lo + v * (vo_stage_bytes(NC) >> 4) + kk * (2048 >> 4),
+                                                idesc_o, (t_b | half | kk) != 0 ? 1u : 0u);
+                            mma_commit(&vo_empty[v]);
+                        }
+                        __syncwarp();
+                        if (++v == VO_STAGES) {
+                            v = 0;
+                            vph ^= 1u;
+                        }
                     }
                     if (!ok) break;
-                    mma_commit(pv_done);
+                    if (leader) mma_commit(pv_done);
+                    __syncwarp();
                     ++t_b;
                 }
                 if (++in_head == per_head) in_head = 0;
             }
-            if (!ok) report_error(a.err_word, abort_flag, DEV_TIMEOUT_VO_MMA);
+            if (!ok && leader) report_error(a.err_word, abort_flag, DEV_TIMEOUT_VO_MMA);
+            __syncwarp();
         }
     } else {
         // ---------------- softmax warps: two per quadrant, 64 keys of a query row each --------

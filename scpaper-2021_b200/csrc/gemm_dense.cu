@@ -105,7 +105,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     float* s_bias = reinterpret_cast<float*>(misc + 256);  // [2][BN]
     int* s_col = reinterpret_cast<int*>(s_bias + 2 * BN);  // [2][BN]
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = uniform_warp_id();
     const int lane = threadIdx.x & 31;
     const int tiles_n = (N + BN - 1) / BN;
     const int tiles_m = (M + BM - 1) / BM;
@@ -215,57 +215,65 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             }
         }
     } else if (warp == 1) {
-        // ---------------- MMA issuer ----------------
-        if (elect_one()) {
-            constexpr uint32_t idesc = make_idesc_f16(BM, Cfg::MMA_N, 0, B_MN ? 1 : 0);
-            int it = 0, tile_iter = 0;
-            bool ok = true;
-            for (int t = blockIdx.x; ok && t < total_tiles; t += gridDim.x, ++tile_iter) {
-                const TileCoord c = decode(t);
-                const int buf = PERSIST ? (tile_iter & 1) : 0;
-                const uint32_t use_ph = PERSIST ? ((tile_iter >> 1) & 1) : (tile_iter & 1);
-                // (an empty K slice issues no MMA: the commit below then arrives at once and the
-                // epilogue writes zeros)
-                // the epilogue must have drained this accumulator's previous tile
-                if (!mbar_wait_bounded(&acc_empty[buf], use_ph ^ 1, abort_flag)) {
-                    report_error(err_word, abort_flag, DEV_TIMEOUT_GEMM_MMA);
+        // ---------------- MMA issuer (warp-uniform, one elected lane issues) ----------------
+        const bool leader = elect_one();
+        constexpr uint32_t idesc = make_idesc_f16(BM, Cfg::MMA_N, 0, B_MN ? 1 : 0);
+        const uint32_t a_base = desc_lo(smem_u32(sA));
+        // MN-major: 16 K-rows = two 8-row groups of 128 bytes (SBO 1024); the next 64-column atom
+        // sits BK * 128 bytes further (LBO).
+        const uint32_t b_base =
+            B_MN ? ((smem_u32(sB) & 0x3FFFFu) >> 4) | (static_cast<uint32_t>(BK * 128 / 16) << 16)
+                 : desc_lo(smem_u32(sB));
+        int s = 0, tile_iter = 0;
+        uint32_t ph = 0;
+        bool ok = true;
+        for (int t = blockIdx.x; ok && t < total_tiles; t += gridDim.x, ++tile_iter) {
+            const TileCoord c = decode(t);
+            const int buf = PERSIST ? (tile_iter & 1) : 0;
+            const uint32_t use_ph = PERSIST ? ((tile_iter >> 1) & 1) : (tile_iter & 1);
+            // (an empty K slice issues no MMA: the commit below then arrives at once and the
+            // epilogue writes zeros)
+            // the epilogue must have drained this accumulator's previous tile
+            if (!mbar_wait_bounded(&acc_empty[buf], use_ph ^ 1, abort_flag)) {
+                ok = false;
+                break;
+            }
+            tc_fence_after_sync();
+            const uint32_t d_tmem = tmem_base + buf * BN;
+            for (int i = 0; i < c.num_kb; ++i) {
+                if (!mbar_wait_bounded(&full_bar[s], ph, abort_flag)) {
+                    ok = false;
                     break;
                 }
                 tc_fence_after_sync();
-                const uint32_t d_tmem = tmem_base + buf * BN;
-                for (int i = 0; i < c.num_kb; ++i, ++it) {
-                    const int s = it % STAGES;
-                    const uint32_t ph = (it / STAGES) & 1;
-                    if (!mbar_wait_bounded(&full_bar[s], ph, abort_flag)) {
-                        report_error(err_word, abort_flag, DEV_TIMEOUT_GEMM_MMA);
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after_sync();
-                    if (it == 0) ET_TL(3);
-                    const uint32_t a_addr = smem_u32(sA + s * A_STAGE_BYTES);
-                    const uint32_t b_addr = smem_u32(sB + s * Cfg::B_STAGE_BYTES);
+                if (tile_iter == 0 && i == 0 && leader) ET_TL(3);
+                const uint32_t a_lo = a_base + s * (A_STAGE_BYTES >> 4);
+                const uint32_t b_lo = b_base + s * (Cfg::B_STAGE_BYTES >> 4);
+                if (leader) {
 #pragma unroll
                     for (int k = 0; k < BK / 16; ++k) {
-                        const uint64_t ad = make_smem_desc(a_addr + k * 32, 16, 1024, SWZ_128B);
-                        // MN-major: 16 K-rows = two 8-row groups of 128 bytes (SBO 1024); the
-                        // next 64-column atom sits BK * 128 bytes further (LBO).
 #pragma unroll
-                        for (int h = 0; h < Cfg::N_HALVES; ++h) {
-                            const uint32_t bh = b_addr + h * (Cfg::MMA_N * 128);
-                            const uint64_t bd =
-                                B_MN ? make_smem_desc(bh + k * 2048, BK * 128, 1024, SWZ_128B)
-                                     : make_smem_desc(bh + k * 32, 16, 1024, SWZ_128B);
-                            mma_f16_ss(d_tmem + h * Cfg::MMA_N, ad, bd, idesc,
-                                       (i | k) != 0 ? 1u : 0u);
-                        }
+                        for (int h = 0; h < Cfg::N_HALVES; ++h)
+                            mma_f16_ss_k128(d_tmem + h * Cfg::MMA_N, a_lo + k * 2,
+                                            b_lo + h * ((Cfg::MMA_N * 128) >> 4) + k * (B_MN ? 2048 >> 4 : 2),
+                                            idesc, (i | k) != 0 ? 1u : 0u);
                     }
                     mma_commit(&empty_bar[s]);
                 }
-                if (ok) mma_commit(&acc_full[buf]);
+                __syncwarp();
+                if (++s == STAGES) {
+                    s = 0;
+                    ph ^= 1u;
+                }
+            }
+            if (ok && leader) {
+                mma_commit(&acc_full[buf]);
                 ET_TL(tile_iter == 0 ? 4 : 5);
             }
+            __syncwarp();
         }
+        if (!ok && leader) report_error(err_word, abort_flag, DEV_TIMEOUT_GEMM_MMA);
+        __syncwarp();
     } else {
         // ---------------- epilogue: TMEM -> registers -> staging -> global ----------------
         const int q = warp & 3;            // TMEM lane quadrant this warp may read

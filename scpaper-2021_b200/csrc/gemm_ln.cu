@@ -77,7 +77,7 @@ gemm_ln_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     float2* s_part = reinterpret_cast<float2*>(s_beta + LN_BN);  // [2 halves][128 rows]
     float2* s_stats = s_part + 2 * BM;                           // [cluster size][128 rows]
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = uniform_warp_id();
     const int lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();   // this CTA's tile along N
     const uint32_t csize = cluster_nctarank();  // = N / 128
@@ -150,30 +150,38 @@ gemm_ln_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             }
         }
     } else if (warp == 1) {
-        // ---------------- MMA issuer ----------------
-        if (elect_one()) {
-            constexpr uint32_t idesc = make_idesc_f16(BM, LN_BN, 0, 0);
-            bool mma_ok = true;
-            for (int i = 0; i < num_kb; ++i) {
-                const int s = i % LN_STAGES;
-                const uint32_t ph = (i / LN_STAGES) & 1;
-                if (!mbar_wait_bounded(&full_bar[s], ph, abort_flag)) {
-                    report_error(g.err_word, abort_flag, DEV_TIMEOUT_GEMM_MMA);
-                    mma_ok = false;
-                    break;
-                }
-                tc_fence_after_sync();
-                const uint32_t a_addr = smem_u32(sA + s * A_STAGE_BYTES);
-                const uint32_t b_addr = smem_u32(sB + s * (LN_BN * BK * 2));
+        // ---------------- MMA issuer (warp-uniform, one elected lane issues) ----------------
+        const bool leader = elect_one();
+        constexpr uint32_t idesc = make_idesc_f16(BM, LN_BN, 0, 0);
+        const uint32_t a_base = desc_lo(smem_u32(sA)), b_base = desc_lo(smem_u32(sB));
+        bool mma_ok = true;
+        int s = 0;
+        uint32_t ph = 0;
+        for (int i = 0; i < num_kb; ++i) {
+            if (!mbar_wait_bounded(&full_bar[s], ph, abort_flag)) {
+                mma_ok = false;
+                break;
+            }
+            tc_fence_after_sync();
+            const uint32_t a_lo = a_base + s * (A_STAGE_BYTES >> 4);
+            const uint32_t b_lo = b_base + s * ((LN_BN * BK * 2) >> 4);
+            if (leader) {
 #pragma unroll
                 for (int k = 0; k < BK / 16; ++k)
-                    mma_f16_ss(tmem_base, make_smem_desc(a_addr + k * 32, 16, 1024, SWZ_128B),
-                               make_smem_desc(b_addr + k * 32, 16, 1024, SWZ_128B), idesc,
-                               (i | k) != 0 ? 1u : 0u);
+                    mma_f16_ss_k128(tmem_base, a_lo + k * 2, b_lo + k * 2, idesc, (i | k) != 0 ? 1u : 0u);
                 mma_commit(&empty_bar[s]);
             }
-            if (mma_ok) mma_commit(acc_full);
+            __syncwarp();
+            if (++s == LN_STAGES) {
+                s = 0;
+                ph ^= 1u;
+            }
         }
+        if (leader) {
+            if (mma_ok) mma_commit(acc_full);
+            else report_error(g.err_word, abort_flag, DEV_TIMEOUT_GEMM_MMA);
+        }
+        __syncwarp();
     } else {
         // ---------------- epilogue, part 1: bias + residual, this CTA's share of the sums ----
         const int et = threadIdx.x - 64;

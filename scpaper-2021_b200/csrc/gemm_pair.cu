@@ -89,7 +89,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     float* s_bias = reinterpret_cast<float*>(misc + 256);  // [2][BN]
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = uniform_warp_id();
     const int lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();
     const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
@@ -205,9 +205,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             }
         }
     } else if (warp == 1) {
-        // ---------------- MMA issuer (leader CTA) ----------------
-        if (rank == 0 && elect_one()) {
+        // ---------------- MMA issuer (leader CTA; warp-uniform, one elected lane issues) --------
+        if (rank == 0) {
+            const bool leader = elect_one();
             constexpr uint32_t idesc = make_idesc_f16(2 * BM, BN, 0, 0);
+            const uint32_t a_base = desc_lo(smem_u32(sA)), b_base = desc_lo(smem_u32(sB));
+            const uint32_t eb0 = smem_u32(empty_bar), eb1 = map_to_cta(eb0, 1);
+            const uint32_t af0 = smem_u32(acc_full), af1 = map_to_cta(af0, 1);
             int s = 0, tile_iter = 0;
             uint32_t ph = 0;
             bool ok = true;
@@ -216,43 +220,44 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 const uint32_t use_ph = (tile_iter >> 1) & 1;
                 // both CTAs' epilogues must have drained this accumulator's previous tile
                 if (PERSIST && !mbar_wait_bounded(&acc_empty[buf], use_ph ^ 1, abort_flag)) {
-                    report_error(err_word, abort_flag, DEV_TIMEOUT_GEMM_MMA);
+                    ok = false;
                     break;
                 }
                 tc_fence_after_sync();
                 const uint32_t d_tmem = tmem_base + buf * BN;
                 for (int i = 0; i < num_kb; ++i) {
                     if (!mbar_wait_bounded(&full_bar[s], ph, abort_flag)) {
-                        report_error(err_word, abort_flag, DEV_TIMEOUT_GEMM_MMA);
                         ok = false;
                         break;
                     }
                     tc_fence_after_sync();
-                    if (tile_iter == 0 && i == 0) ET_TL(5);
-                    const uint32_t a_addr = smem_u32(sA + s * A_STAGE_BYTES);
-                    const uint32_t b_addr = smem_u32(sB + s * Cfg::B_HALF_BYTES);
+                    if (tile_iter == 0 && i == 0 && leader) ET_TL(5);
+                    const uint32_t a_lo = a_base + s * (A_STAGE_BYTES >> 4);
+                    const uint32_t b_lo = b_base + s * (Cfg::B_HALF_BYTES >> 4);
+                    if (leader) {
 #pragma unroll
-                    for (int k = 0; k < BK / 16; ++k) {
-                        const uint64_t ad = make_smem_desc(a_addr + k * 32, 16, 1024, SWZ_128B);
-                        const uint64_t bd = make_smem_desc(b_addr + k * 32, 16, 1024, SWZ_128B);
-                        mma_f16_ss_pair(d_tmem, ad, bd, idesc, (i | k) != 0 ? 1u : 0u);
+                        for (int k = 0; k < BK / 16; ++k)
+                            mma_f16_ss_pair_k128(d_tmem, a_lo + k * 2, b_lo + k * 2, idesc,
+                                                 (i | k) != 0 ? 1u : 0u);
+                        // the stage is free in both CTAs once these products have read it
+                        mma_commit_pair(eb0 + s * 8);
+                        mma_commit_pair(eb1 + s * 8);
                     }
-                    // the stage is free in both CTAs once these products have read it
-                    const uint32_t eb = smem_u32(&empty_bar[s]);
-                    mma_commit_pair(eb);
-                    mma_commit_pair(map_to_cta(eb, 1));
+                    __syncwarp();
                     if (++s == STAGES) {
                         s = 0;
                         ph ^= 1u;
                     }
                 }
-                if (ok) {
-                    const uint32_t af = smem_u32(&acc_full[buf]);
-                    mma_commit_pair(af);
-                    mma_commit_pair(map_to_cta(af, 1));
+                if (ok && leader) {
+                    mma_commit_pair(af0 + buf * 8);
+                    mma_commit_pair(af1 + buf * 8);
                     ET_TL(6);
                 }
+                __syncwarp();
             }
+            if (!ok && leader) report_error(err_word, abort_flag, DEV_TIMEOUT_GEMM_MMA);
+            __syncwarp();
         }
     } else {
         // ---------------- epilogue of this CTA's 128 rows ----------------

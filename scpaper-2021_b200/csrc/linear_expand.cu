@@ -194,7 +194,7 @@ linear_expand_kernel(const __grid_constant__ CUtensorMap tmX, const ExpandArgs g
     int* s_ptr = reinterpret_cast<int*>(s_bias + BN);             // CSR: [BN + 1] row starts
     int* s_dup = s_ptr + X_ROW_LIST;                              // CSR: [BN] row holds duplicates
 
-    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);  // (known to be warp-uniform)
+    const int warp = uniform_warp_id();
     const int lane = threadIdx.x & 31;
     const int n0 = static_cast<int>(blockIdx.x / g.groups) * BN;
     const int m0 = static_cast<int>(blockIdx.x % g.groups) * g.mb * BM;

@@ -82,7 +82,7 @@ qkv_attention_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
     float* s_bias = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + 256);  // [192]
     float* s_x = s_bias + 192;  // max exchange [2][128], sum exchange [2][128]
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = uniform_warp_id();
     const int lane = threadIdx.x & 31;
     const int h = blockIdx.x;
     const int b = blockIdx.y;
@@ -178,67 +178,72 @@ qkv_attention_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
             }
         }
     } else if (warp == 1) {
-        // ---------------- MMA issuer ----------------
-        if (elect_one()) {
-            constexpr uint32_t idesc_p = make_idesc_f16(128, 192, 0, 0);
-            constexpr uint32_t idesc_s = make_idesc_f16(128, 128, 0, 0);
-            constexpr uint32_t idesc_o = make_idesc_f16(128, 64, 0, 1);  // V is MN-major
-            int s = 0;
-            uint32_t ph = 0;
-            bool ok = true;
-            for (int i = 0; i < nkb; ++i) {
-                if (!mbar_wait_bounded(&full_bar[s], ph, abort_flag)) {
-                    report_error(a.err_word, abort_flag, DEV_TIMEOUT_ATTN_MMA);
-                    ok = false;
-                    break;
-                }
-                tc_fence_after_sync();
-                if (i == 0) QA_TL(4);
-                const uint32_t a_addr = smem_u32(smem + s * QA_STAGE);
-                const uint32_t b_addr = a_addr + QA_ATOM;
+        // ---------------- MMA issuer (warp-uniform, one elected lane issues) ----------------
+        const bool leader = elect_one();
+        constexpr uint32_t idesc_p = make_idesc_f16(128, 192, 0, 0);
+        constexpr uint32_t idesc_s = make_idesc_f16(128, 128, 0, 0);
+        constexpr uint32_t idesc_o = make_idesc_f16(128, 64, 0, 1);  // V is MN-major
+        const uint32_t ring = desc_lo(smem_u32(smem));
+        int s = 0;
+        uint32_t ph = 0;
+        bool ok = true;
+        for (int i = 0; i < nkb; ++i) {
+            if (!mbar_wait_bounded(&full_bar[s], ph, abort_flag)) {
+                ok = false;
+                break;
+            }
+            tc_fence_after_sync();
+            if (i == 0 && leader) QA_TL(4);
+            const uint32_t a_lo = ring + s * (QA_STAGE >> 4);
+            const uint32_t b_lo = a_lo + (QA_ATOM >> 4);
+            if (leader) {
 #pragma unroll
                 for (int k = 0; k < 4; ++k)
-                    mma_f16_ss(tmem_base, make_smem_desc(a_addr + k * 32, 16, 1024, SWZ_128B),
-                               make_smem_desc(b_addr + k * 32, 16, 1024, SWZ_128B), idesc_p,
-                               (i | k) != 0 ? 1u : 0u);
+                    mma_f16_ss_k128(tmem_base, a_lo + k * 2, b_lo + k * 2, idesc_p, (i | k) != 0 ? 1u : 0u);
                 mma_commit(&empty_bar[s]);
-                if (++s == QA_STAGES) {
-                    s = 0;
-                    ph ^= 1u;
-                }
             }
-            if (ok) {
-                mma_commit(proj_full);
-                QA_TL(5);
-                ok = mbar_wait_bounded(qkv_ready, 0, abort_flag);
-                if (!ok) report_error(a.err_word, abort_flag, DEV_TIMEOUT_ATTN_MMA);
-            }
-            if (ok) {
-                tc_fence_after_sync();
-                const uint32_t q_addr = smem_u32(sQ), k_addr = smem_u32(sK), v_addr = smem_u32(sV),
-                               p_addr = smem_u32(sP);
-#pragma unroll
-                for (int kk = 0; kk < 4; ++kk)
-                    mma_f16_ss(tmem_S, make_smem_desc(q_addr + kk * 32, 16, 1024, SWZ_128B),
-                               make_smem_desc(k_addr + kk * 32, 16, 1024, SWZ_128B), idesc_s,
-                               kk != 0 ? 1u : 0u);
-                mma_commit(s_full);
-                ok = mbar_wait_bounded(p_full, 0, abort_flag);
-                if (!ok) report_error(a.err_word, abort_flag, DEV_TIMEOUT_ATTN_MMA);
-                if (ok) {
-                    tc_fence_after_sync();
-#pragma unroll
-                    for (int kk = 0; kk < 8; ++kk) {
-                        const uint32_t p_off = (kk >> 2) * QA_ATOM + (kk & 3) * 32;
-                        // V tile: 16 keys = two groups of 8 rows of 128 bytes (SBO = 1024)
-                        mma_f16_ss(tmem_O, make_smem_desc(p_addr + p_off, 16, 1024, SWZ_128B),
-                                   make_smem_desc(v_addr + kk * 2048, QA_ATOM, 1024, SWZ_128B),
-                                   idesc_o, kk != 0 ? 1u : 0u);
-                    }
-                    mma_commit(o_full);
-                }
+            __syncwarp();
+            if (++s == QA_STAGES) {
+                s = 0;
+                ph ^= 1u;
             }
         }
+        if (ok) {
+            if (leader) {
+                mma_commit(proj_full);
+                QA_TL(5);
+            }
+            __syncwarp();
+            ok = mbar_wait_bounded(qkv_ready, 0, abort_flag);
+        }
+        if (ok) {
+            tc_fence_after_sync();
+            const uint32_t q_lo = desc_lo(smem_u32(sQ)), k_lo = desc_lo(smem_u32(sK)),
+                           p_lo = desc_lo(smem_u32(sP));
+            const uint32_t v_lo = ((smem_u32(sV) & 0x3FFFFu) >> 4) | (static_cast<uint32_t>(QA_ATOM >> 4) << 16);
+            if (leader) {
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk)
+                    mma_f16_ss_k128(tmem_S, q_lo + kk * 2, k_lo + kk * 2, idesc_s, kk != 0 ? 1u : 0u);
+                mma_commit(s_full);
+            }
+            __syncwarp();
+            ok = mbar_wait_bounded(p_full, 0, abort_flag);
+            if (ok) {
+                tc_fence_after_sync();
+                if (leader) {
+#pragma unroll
+                    for (int kk = 0; kk < 8; ++kk)
+                        // V tile: 16 keys = two groups of 8 rows of 128 bytes (SBO = 1024)
+                        mma_f16_ss_k128(tmem_O, p_lo + (kk >> 2) * (QA_ATOM >> 4) + (kk & 3) * 2,
+                                        v_lo + kk * (2048 >> 4), idesc_o, kk != 0 ? 1u : 0u);
+                    mma_commit(o_full);
+                }
+                __syncwarp();
+            }
+        }
+        if (!ok && leader) report_error(a.err_word, abort_flag, DEV_TIMEOUT_ATTN_MMA);
+        __syncwarp();
     } else {
         // ---------------- conversion, softmax, output ----------------
         const int qd = warp & 3;         // tensor-memory lane quadrant
