@@ -98,14 +98,82 @@ def _p(t):
     return None if t is None else c_void_p(t.data_ptr())
 
 
+def _a(t):
+    """Address of a tensor as a plain integer, for _call (whose argument types are declared)."""
+    return None if t is None else t.data_ptr()
+
+
 def _stream():
-    import torch
-    return c_void_p(torch.cuda.current_stream().cuda_stream)
+    return c_void_p(_raw_stream())
+
+
+def _raw_stream() -> int:
+    """Handle of the current stream of the current device (torch.cuda.current_stream() builds a
+    Stream object: 3 us a call, as much as the launch it serves)."""
+    return _torch_c()._cuda_getCurrentRawStream(_torch_c()._cuda_getDevice())
+
+
+_torch_c_module = None
+
+
+def _torch_c():
+    global _torch_c_module
+    if _torch_c_module is None:
+        import torch
+        _torch_c_module = torch._C
+    return _torch_c_module
 
 
 def _empty(shape, like):
     import torch
+    if like.dtype is torch.float16:
+        return like.new_empty(shape)
     return torch.empty(shape, dtype=torch.float16, device=like.device)
+
+
+# Argument kinds of the calls made per forward pass: p = pointer, i = int, z = size_t, f = float.
+# Declared once, so that plain integers are converted natively instead of through a ctypes object
+# per argument.
+_SIGNATURES = {
+    "et_linear_dense_fwd": "ppppiiiip",
+    "et_linear_tile_fwd": "pppippp" "iiiip",
+    "et_linear_tile_packed_fwd": "ppppippp" "iiiip",
+    "et_linear_row_fwd": "ppippp" "iiiip",
+    "et_linear_row_compressed_fwd": "ppippp" "iip",
+    "et_linear_col_fwd": "ppippp" "iiiipzp",
+    "et_linear_col_noalloc_fwd": "ppippp" "iiiip",
+    "et_linear_1x16_fwd": "pppippp" "iiiip",
+    "et_linear_csr_fwd": "pppippp" "iiiip",
+    "et_skip_layernorm_fwd": "pppppiip",
+    "et_linear_skip_layernorm_fwd": "ppppppp" "iiip",
+    "et_layernorm_fwd": "ppppiip",
+    "et_act_fwd": "ppzip",
+    "et_bias_add_fwd": "ppiip",
+    "et_attention_fwd": "pppp" "iiiiiiiiii" "ppfp",
+    "et_qkv_attention_fwd": "pppp" "iiiiiii" "ppfp",
+    "et_attention_pruned_v_fwd": "pppppip" "iiiiiiiii" "ppfp",
+    "et_attention_fuse_o_fwd": "ppppp" "pppipp" "iiiiiiiiii" "pfp",
+    "et_attention_fuse_o_single_launch_fwd": "ppppp" "pppipp" "iiiiiiiiii" "pfp",
+    "et_linear_vo_fwd": "ppppiiiip",
+    "et_linear_vo_pruned_fwd": "ppppiiiiip",
+    "et_fused_vo_attention_fwd": "ppppp" "iiiiiiii" "ppfp",
+    "et_fused_vo_attention_pruned_fwd": "ppppippp" "iiiiiiii" "ppfp",
+    "et_encoder_layer_fwd": "pppiii" "pppzp",
+}
+_KINDS = {"p": c_void_p, "i": c_int, "z": c_size_t, "f": c_float}
+_calls = {}
+
+
+def _call(name: str, *args) -> None:
+    """One forward entry point with plain Python arguments; raises on a status."""
+    fn = _calls.get(name)
+    if fn is None or fn[0] is not _lib:
+        proto = ctypes.CFUNCTYPE(c_int, *[_KINDS[k] for k in _SIGNATURES[name]])
+        fn = (lib(), proto((name, lib())))
+        _calls[name] = fn
+    status = fn[1](*args)
+    if status != 0:
+        check(status, name)
 
 
 # ---- Linear layers ------------------------------------------------------------------------
@@ -115,8 +183,7 @@ def linear_dense(x, w, bias=None, act=ACT_NONE, out=None):
     T, inn = x.shape
     y = _empty((T, w.shape[0]), x) if out is None else out
     out = w.shape[0]
-    check(lib().et_linear_dense_fwd(_p(x), _p(w), _p(bias), _p(y), c_int(T), c_int(inn),
-                                    c_int(out), c_int(act), _stream()), "et_linear_dense_fwd")
+    _call("et_linear_dense_fwd", _a(x), _a(w), _a(bias), _a(y), T, inn, out, act, _raw_stream())
     return y
 
 
@@ -124,10 +191,8 @@ def linear_tile(x, row_ptr, row_off, tiles, out, bias=None, act=ACT_NONE):
     T, inn = x.shape
     y = _empty((T, out), x)
     nnz = int(tiles.shape[0]) if tiles is not None else 0
-    check(lib().et_linear_tile_fwd(_p(row_ptr), _p(row_off) if nnz else None,
-                                   _p(tiles) if nnz else None, c_int(nnz), _p(bias), _p(x), _p(y),
-                                   c_int(T), c_int(inn), c_int(out), c_int(act), _stream()),
-          "et_linear_tile_fwd")
+    _call("et_linear_tile_fwd", _a(row_ptr), _a(row_off) if nnz else None,
+          _a(tiles) if nnz else None, nnz, _a(bias), _a(x), _a(y), T, inn, out, act, _raw_stream())
     return y
 
 
@@ -189,11 +254,9 @@ def tile_densify(row_ptr, row_off, tiles, inn: int, out: int):
 def linear_tile_packed(x, pk: "PackedTiles", bias=None, act=ACT_NONE):
     T, inn = x.shape
     y = _empty((T, pk.out), x)
-    check(lib().et_linear_tile_packed_fwd(_p(pk.row_ptr), _p(pk.pk_mask), _p(pk.pk_off),
-                                          _p(pk.tiles) if pk.nnz else None, c_int(pk.nnz),
-                                          _p(bias), _p(x), _p(y), c_int(T), c_int(inn),
-                                          c_int(pk.out), c_int(act), _stream()),
-          "et_linear_tile_packed_fwd")
+    _call("et_linear_tile_packed_fwd", _a(pk.row_ptr), _a(pk.pk_mask), _a(pk.pk_off),
+          _a(pk.tiles) if pk.nnz else None, pk.nnz, _a(bias), _a(x), _a(y), T, inn, pk.out, act,
+          _raw_stream())
     return y
 
 
@@ -201,9 +264,8 @@ def linear_row(x, row_id, rows, out, bias=None, act=ACT_NONE):
     T, inn = x.shape
     y = _empty((T, out), x)
     nn = 0 if row_id is None else int(row_id.shape[0])
-    check(lib().et_linear_row_fwd(_p(row_id) if nn else None, _p(rows) if nn else None, c_int(nn),
-                                  _p(bias), _p(x), _p(y), c_int(T), c_int(inn), c_int(out),
-                                  c_int(act), _stream()), "et_linear_row_fwd")
+    _call("et_linear_row_fwd", _a(row_id) if nn else None, _a(rows) if nn else None, nn, _a(bias),
+          _a(x), _a(y), T, inn, out, act, _raw_stream())
     return y
 
 
@@ -211,9 +273,8 @@ def linear_row_compressed(x, row_id, rows, bias=None):
     T, inn = x.shape
     nn = int(row_id.shape[0])
     y = _empty((T, nn), x)
-    check(lib().et_linear_row_compressed_fwd(_p(row_id), _p(rows), c_int(nn), _p(bias), _p(x),
-                                             _p(y), c_int(T), c_int(inn), _stream()),
-          "et_linear_row_compressed_fwd")
+    _call("et_linear_row_compressed_fwd", _a(row_id), _a(rows), nn, _a(bias), _a(x), _a(y), T, inn,
+          _raw_stream())
     return y
 
 
@@ -223,9 +284,8 @@ def linear_col(x, col_id, cols, bias=None, act=ACT_NONE, scratch=None):
     y = _empty((T, out), x)
     if scratch is None:
         scratch = _empty((T, nn), x)
-    check(lib().et_linear_col_fwd(_p(col_id), _p(cols), c_int(nn), _p(bias), _p(x), _p(y),
-                                  c_int(T), c_int(inn), c_int(out), c_int(act), _p(scratch),
-                                  c_size_t(scratch.numel() * 2), _stream()), "et_linear_col_fwd")
+    _call("et_linear_col_fwd", _a(col_id), _a(cols), nn, _a(bias), _a(x), _a(y), T, inn, out, act,
+          _a(scratch), scratch.numel() * 2, _raw_stream())
     return y
 
 
@@ -234,9 +294,8 @@ def linear_col_noalloc(x, col_id, cols, y, bias=None, act=ACT_NONE):
     the caller supplies the output tensor too, so nothing is allocated here either."""
     T, inn = x.shape
     out, nn = cols.shape
-    check(lib().et_linear_col_noalloc_fwd(_p(col_id), _p(cols), c_int(nn), _p(bias), _p(x), _p(y),
-                                          c_int(T), c_int(inn), c_int(out), c_int(act),
-                                          _stream()), "et_linear_col_noalloc_fwd")
+    _call("et_linear_col_noalloc_fwd", _a(col_id), _a(cols), nn, _a(bias), _a(x), _a(y), T, inn,
+          out, act, _raw_stream())
     return y
 
 
@@ -244,10 +303,8 @@ def linear_1x16(x, tile_idx, row_idx, data, out, bias=None, act=ACT_NONE):
     T, inn = x.shape
     y = _empty((T, out), x)
     nvec = 0 if row_idx is None else int(row_idx.shape[0])
-    check(lib().et_linear_1x16_fwd(_p(tile_idx), _p(row_idx) if nvec else None,
-                                   _p(data) if nvec else None, c_int(nvec), _p(bias), _p(x), _p(y),
-                                   c_int(T), c_int(inn), c_int(out), c_int(act), _stream()),
-          "et_linear_1x16_fwd")
+    _call("et_linear_1x16_fwd", _a(tile_idx), _a(row_idx) if nvec else None,
+          _a(data) if nvec else None, nvec, _a(bias), _a(x), _a(y), T, inn, out, act, _raw_stream())
     return y
 
 
@@ -273,10 +330,8 @@ def linear_csr(x, indptr, indices, data, out, bias=None, act=ACT_NONE):
     T, inn = x.shape
     y = _empty((T, out), x)
     nnz = 0 if indices is None else int(indices.shape[0])
-    check(lib().et_linear_csr_fwd(_p(indptr), _p(indices) if nnz else None,
-                                  _p(data) if nnz else None, c_int(nnz), _p(bias), _p(x), _p(y),
-                                  c_int(T), c_int(inn), c_int(out), c_int(act), _stream()),
-          "et_linear_csr_fwd")
+    _call("et_linear_csr_fwd", _a(indptr), _a(indices) if nnz else None, _a(data) if nnz else None,
+          nnz, _a(bias), _a(x), _a(y), T, inn, out, act, _raw_stream())
     return y
 
 
@@ -285,8 +340,8 @@ def linear_csr(x, indptr, indices, data, out, bias=None, act=ACT_NONE):
 def skip_layernorm(src, skip, gamma, beta, out=None):
     rows, size = src.shape
     out = _empty((rows, size), src) if out is None else out
-    check(lib().et_skip_layernorm_fwd(_p(src), _p(skip), _p(gamma), _p(beta), _p(out), c_int(rows),
-                                      c_int(size), _stream()), "et_skip_layernorm_fwd")
+    _call("et_skip_layernorm_fwd", _a(src), _a(skip), _a(gamma), _a(beta), _a(out), rows, size,
+          _raw_stream())
     return out
 
 
@@ -295,31 +350,27 @@ def linear_skip_layernorm(x, w, bias, resid, gamma, beta, out=None):
     T, inn = x.shape
     n = w.shape[0]
     y = _empty((T, n), x) if out is None else out
-    check(lib().et_linear_skip_layernorm_fwd(_p(x), _p(w), _p(bias), _p(resid), _p(gamma),
-                                             _p(beta), _p(y), c_int(T), c_int(inn), c_int(n),
-                                             _stream()), "et_linear_skip_layernorm_fwd")
+    _call("et_linear_skip_layernorm_fwd", _a(x), _a(w), _a(bias), _a(resid), _a(gamma), _a(beta),
+          _a(y), T, inn, n, _raw_stream())
     return y
 
 
 def layernorm(src, gamma, beta):
     rows, size = src.shape
     out = _empty((rows, size), src)
-    check(lib().et_layernorm_fwd(_p(src), _p(gamma), _p(beta), _p(out), c_int(rows), c_int(size),
-                                 _stream()), "et_layernorm_fwd")
+    _call("et_layernorm_fwd", _a(src), _a(gamma), _a(beta), _a(out), rows, size, _raw_stream())
     return out
 
 
 def act(x, kind, inplace=False):
     out = x if inplace else _empty(tuple(x.shape), x)
-    check(lib().et_act_fwd(_p(x), _p(out), c_size_t(x.numel()), c_int(kind), _stream()),
-          "et_act_fwd")
+    _call("et_act_fwd", _a(x), _a(out), x.numel(), kind, _raw_stream())
     return out
 
 
 def bias_add_(data, bias):
     rows, cols = data.shape
-    check(lib().et_bias_add_fwd(_p(data), _p(bias), c_int(rows), c_int(cols), _stream()),
-          "et_bias_add_fwd")
+    _call("et_bias_add_fwd", _a(data), _a(bias), rows, cols, _raw_stream())
     return data
 
 
@@ -334,10 +385,8 @@ def attention(q, k, v, batch, seq, nhead, dh_qk, dh_v, mask_kind=MASK_NONE, mask
     ldv = v.stride(0) if ldv is None else ldv
     z = _empty((batch * seq, nhead * dh_v), q) if out is None else out
     scale = (1.0 / dh_qk ** 0.5) if scale is None else scale
-    check(lib().et_attention_fwd(_p(q), _p(k), _p(v), _p(z), c_int(batch), c_int(seq),
-                                 c_int(nhead), c_int(dh_qk), c_int(dh_v), c_int(ldq), c_int(ldk),
-                                 c_int(ldv), c_int(nhead * dh_v), c_int(mask_kind), _p(mask),
-                                 _p(valid_len), c_float(scale), _stream()), "et_attention_fwd")
+    _call("et_attention_fwd", _a(q), _a(k), _a(v), _a(z), batch, seq, nhead, dh_qk, dh_v, ldq, ldk,
+          ldv, nhead * dh_v, mask_kind, _a(mask), _a(valid_len), scale, _raw_stream())
     return z
 
 
@@ -346,10 +395,8 @@ def qkv_attention(x, wqkv, bqkv, batch, seq, nhead, kdim, vdim, mask_kind=MASK_N
     """Fused Q/K/V projection + attention (seq <= 128, 64-wide heads)."""
     z = _empty((batch * seq, vdim), x)
     scale = (1.0 / (kdim // nhead) ** 0.5) if scale is None else scale
-    check(lib().et_qkv_attention_fwd(_p(x), _p(wqkv), _p(bqkv), _p(z), c_int(batch), c_int(seq),
-                                     c_int(x.shape[1]), c_int(nhead), c_int(kdim), c_int(vdim),
-                                     c_int(mask_kind), _p(mask), _p(valid_len), c_float(scale),
-                                     _stream()), "et_qkv_attention_fwd")
+    _call("et_qkv_attention_fwd", _a(x), _a(wqkv), _a(bqkv), _a(z), batch, seq, x.shape[1], nhead,
+          kdim, vdim, mask_kind, _a(mask), _a(valid_len), scale, _raw_stream())
     return z
 
 
@@ -357,13 +404,9 @@ def attention_pruned_v(q, k, vc, col_id, head_ptr, batch, seq, nhead, dh_qk, dh_
                        mask_kind=MASK_NONE, mask=None, valid_len=None, scale=None):
     z = _empty((batch * seq, nhead * dh_v), q)
     scale = (1.0 / dh_qk ** 0.5) if scale is None else scale
-    check(lib().et_attention_pruned_v_fwd(_p(q), _p(k), _p(vc), _p(col_id), _p(head_ptr),
-                                          c_int(int(col_id.shape[0])), _p(z), c_int(batch),
-                                          c_int(seq), c_int(nhead), c_int(dh_qk), c_int(dh_v),
-                                          c_int(q.stride(0)), c_int(k.stride(0)),
-                                          c_int(nhead * dh_v), c_int(mask_kind), _p(mask),
-                                          _p(valid_len), c_float(scale), _stream()),
-          "et_attention_pruned_v_fwd")
+    _call("et_attention_pruned_v_fwd", _a(q), _a(k), _a(vc), _a(col_id), _a(head_ptr),
+          col_id.shape[0], _a(z), batch, seq, nhead, dh_qk, dh_v, q.stride(0), k.stride(0),
+          nhead * dh_v, mask_kind, _a(mask), _a(valid_len), scale, _raw_stream())
     return z
 
 
@@ -389,8 +432,8 @@ def attention_fuse_o(q, k, v, o_row_ptr, o_row_off, o_tiles, o_bias, batch, seq,
 
 def linear_vo(x, w_vo, bias, batch, seq, nhead, emdim):
     vo = _empty((batch * nhead * seq, emdim), x)
-    check(lib().et_linear_vo_fwd(_p(x), _p(w_vo), _p(bias), _p(vo), c_int(batch), c_int(seq),
-                                 c_int(nhead), c_int(emdim), _stream()), "et_linear_vo_fwd")
+    _call("et_linear_vo_fwd", _a(x), _a(w_vo), _a(bias), _a(vo), batch, seq, nhead, emdim,
+          _raw_stream())
     return vo
 
 
@@ -398,12 +441,9 @@ def fused_vo_attention(q, k, vo, bias_o, batch, seq, nhead, dh_qk, emdim, mask_k
                        mask=None, valid_len=None, scale=None):
     out = _empty((batch * seq, emdim), q)
     scale = (1.0 / dh_qk ** 0.5) if scale is None else scale
-    check(lib().et_fused_vo_attention_fwd(_p(q), _p(k), _p(vo), _p(bias_o), _p(out), c_int(batch),
-                                          c_int(seq), c_int(nhead), c_int(dh_qk), c_int(emdim),
-                                          c_int(q.stride(0)), c_int(k.stride(0)),
-                                          c_int(mask_kind), _p(mask), _p(valid_len),
-                                          c_float(scale), _stream()),
-          "et_fused_vo_attention_fwd")
+    _call("et_fused_vo_attention_fwd", _a(q), _a(k), _a(vo), _a(bias_o), _a(out), batch, seq, nhead,
+          dh_qk, emdim, q.stride(0), k.stride(0), mask_kind, _a(mask), _a(valid_len), scale,
+          _raw_stream())
     return out
 
 
@@ -413,9 +453,8 @@ def linear_vo_pruned(x, w_vo_c, bias, batch, seq, nhead, emdim):
     """w_vo_c: [nhead, emdim, nnz_col]; returns VOc [batch * nhead * seq, nnz_col]."""
     nnz = int(w_vo_c.shape[2])
     vo = _empty((batch * nhead * seq, nnz), x)
-    check(lib().et_linear_vo_pruned_fwd(_p(x), _p(w_vo_c), _p(bias), _p(vo), c_int(batch), c_int(seq),
-                                        c_int(nhead), c_int(emdim), c_int(nnz), _stream()),
-          "et_linear_vo_pruned_fwd")
+    _call("et_linear_vo_pruned_fwd", _a(x), _a(w_vo_c), _a(bias), _a(vo), batch, seq, nhead, emdim,
+          nnz, _raw_stream())
     return vo
 
 
@@ -425,11 +464,9 @@ def fused_vo_attention_pruned(q, k, vo_c, col_id, bias_o, batch, seq, nhead, dh_
     scratch = _empty((batch * seq, nnz), q)
     out = _empty((batch * seq, emdim), q)
     scale = (1.0 / dh_qk ** 0.5) if scale is None else scale
-    check(lib().et_fused_vo_attention_pruned_fwd(
-        _p(q), _p(k), _p(vo_c), _p(col_id), c_int(nnz), _p(bias_o), _p(scratch), _p(out),
-        c_int(batch), c_int(seq), c_int(nhead), c_int(dh_qk), c_int(emdim), c_int(q.stride(0)),
-        c_int(k.stride(0)), c_int(mask_kind), _p(mask), _p(valid_len), c_float(scale), _stream()),
-        "et_fused_vo_attention_pruned_fwd")
+    _call("et_fused_vo_attention_pruned_fwd", _a(q), _a(k), _a(vo_c), _a(col_id), nnz, _a(bias_o),
+          _a(scratch), _a(out), batch, seq, nhead, dh_qk, emdim, q.stride(0), k.stride(0),
+          mask_kind, _a(mask), _a(valid_len), scale, _raw_stream())
     return out
 
 
@@ -564,11 +601,9 @@ class EncoderLayer:
 
     def forward(self, x, out, batch, seq, workspace, mask_kind=MASK_NONE, mask=None,
                 valid_len=None):
-        check(lib().et_encoder_layer_fwd(ctypes.byref(self.desc), _p(x), _p(out), c_int(batch),
-                                         c_int(seq), c_int(mask_kind), _p(mask), _p(valid_len),
-                                         _p(workspace), c_size_t(workspace.numel() *
-                                                                 workspace.element_size()),
-                                         _stream()), "et_encoder_layer_fwd")
+        _call("et_encoder_layer_fwd", ctypes.byref(self.desc), _a(x), _a(out), batch, seq,
+              mask_kind, _a(mask), _a(valid_len), _a(workspace),
+              workspace.numel() * workspace.element_size(), _raw_stream())
         return out
 
 
