@@ -57,6 +57,49 @@ int ln_fusion_mask(int T, int hidden) {
     return et_linear_skip_layernorm_pays(T, hidden, hidden) ? 3 : 0;
 }
 
+// How a dense [T, K] x [hidden, K]^T product followed by residual + LayerNorm runs with few row blocks:
+// tiles of 32 to 128 columns and K slices (gemm_narrow.cu), added up by the LayerNorm that follows.
+// splits = 0: the fused kernel (gemm_ln.cu) is expected to be faster.  Estimates in SM cycles, from
+// timelines on B200: a K block costs its bytes at 84 per cycle, which is also what bounds the fused
+// kernel's hidden / 128 CTAs per row block (390 cycles a block, and 5700 from the last product to
+// the end); a second launch costs its hand-over (1700) and one L2 round trip with the slices' traffic.
+struct NarrowPlan {
+    int bn, splits;
+};
+int g_narrow_ln = -1;  // test hook: 0 = never
+NarrowPlan pick_narrow_ln(int T, int hidden, int K) {
+    NarrowPlan p = {0, 0};
+    if (g_narrow_ln == 0 || g_ln_fusion >= 0 || g_force_splits != 0 || hidden > 2048 || hidden % 8) return p;
+    const long sms = sm_count() > 0 ? sm_count() : 148;
+    const long mt = (T + 127) / 128, nkb = (K + 63) / 64;
+    long best = nkb * 390 + 900 + 5700;
+    if (!et_linear_skip_layernorm_pays(T, K, hidden)) best += 2500;
+    best = best * 9 / 10;  // (within a tenth the two tie)
+    for (int bn : {32, 64, 128})
+        for (int s = 1; s <= kMaxSplits && nkb >= 2 * s; ++s) {
+            if (mt * ((hidden + bn - 1) / bn) * s > sms) continue;
+            const long gemm = 1350 + (nkb + s - 1) / s * ((16384 + bn * 128) / 84) + 500 + 12 * bn;
+            const long ln = 1700 + 2000 + static_cast<long>(T) * hidden * 4 * s / (sms * 45);
+            if (gemm + ln < best) {
+                best = gemm + ln;
+                p.bn = bn;
+                p.splits = s;
+            }
+        }
+    return p;
+}
+
+// out = LN(X W^T + bias + resid) for dense W through the narrow tiles.
+int narrow_linear_ln(const NarrowPlan& p, const __half* X, int K, const __half* W, const __half* bias,
+                     const __half* resid, const __half* gamma, const __half* beta, __half* out, float* part,
+                     int T, int hidden, cudaStream_t s) {
+    const int st = launch_gemm_narrow(X, K, W, K, nullptr, part, hidden, T, hidden, K, ET_ACT_NONE, p.bn,
+                                      p.splits, true, s);
+    if (st != ET_OK) return st;
+    return launch_skip_layernorm_partials(part, p.splits, static_cast<size_t>(T) * hidden, bias, resid, gamma,
+                                          beta, out, T, hidden, s);
+}
+
 // Split-K on CTA pairs: 256 x 256 pair tiles, as many K slices as SM pairs allow.  Returns 0
 // when the pair form does not apply.  Measured on B200 at BERT-base sizes the fp32 partial
 // sums (written by the GEMM, re-read by the LayerNorm) cost more than the better machine fill
@@ -190,6 +233,12 @@ int ffn_block(const et_encoder_layer_t* layer, const LayerBuffers& b, int T, __h
     } else if ((st = run_linear(layer->ffn1, b.y, b.f, T, layer->act, b, s)) != ET_OK) {
         return st;
     }
+    const NarrowPlan narrow = ffn2_dense ? pick_narrow_ln(T, layer->hidden, k2) : NarrowPlan{0, 0};
+    if (narrow.splits > 0)
+        return narrow_linear_ln(narrow, b.f, k2, w2, reinterpret_cast<const __half*>(layer->ffn2.bias), b.y,
+                                reinterpret_cast<const __half*>(layer->ln2_gamma),
+                                reinterpret_cast<const __half*>(layer->ln2_beta), out_h, b.part, T,
+                                layer->hidden, s);
     if ((ln_fused & 2) && ffn2_dense && gemm_ln_applies(T, layer->hidden, k2) &&
         reinterpret_cast<const __half*>(out) != b.y) {
         // FFN2, residual and LayerNorm in one kernel
@@ -257,6 +306,8 @@ void et_debug_force_ffn2_splits(int n) { et::g_force_splits = n; }
 // Test hook: 0 = never fuse the Q/K/V projection into the attention kernel.
 void et_debug_set_qkv_fusion(int on) { et::g_qkv_fusion = on != 0; }
 void et_debug_set_ln_fusion(int mode) { et::g_ln_fusion = mode; }
+// Test hook: 0 = never the narrow tiles with K slices in front of a LayerNorm, -1 = automatic.
+void et_debug_set_narrow_ln(int mode) { et::g_narrow_ln = mode; }
 #endif  // ET_TEST_HOOKS
 
 size_t et_encoder_layer_workspace_bytes(const et_encoder_layer_t* layer, int batch, int seq) {
@@ -283,8 +334,10 @@ int et_encoder_layer_fwd(const et_encoder_layer_t* layer, const et_half* x, et_h
     const int dh_qk = layer->kdim / layer->nhead, dh_v = layer->vdim / layer->nhead;
 
     // The fused kernel projects a full 128-token block per sequence whatever its length: below
-    // 96 tokens the padding costs more than the fusion saves (measured at 64: 4 % slower).
-    if (et::g_qkv_fusion && layer->qkv.format == ET_FMT_DENSE && seq >= 96 &&
+    // 96 tokens the padding costs more than the fusion saves (measured at 64: 4 % slower), unless
+    // every CTA has an SM of its own.
+    if (et::g_qkv_fusion && layer->qkv.format == ET_FMT_DENSE &&
+        (seq >= 96 || static_cast<long>(batch) * layer->nhead <= et::sm_count()) &&
         et::qkv_attention_applies(seq, layer->nhead, layer->kdim, layer->vdim)) {
         // short sequences, 64-wide heads: projection and attention in one kernel, the projected
         // Q / K / V never leave the SM
@@ -305,7 +358,18 @@ int et_encoder_layer_fwd(const et_encoder_layer_t* layer, const et_half* x, et_h
             return st;
     }
     const int ln_fused = et::ln_fusion_mask(T, layer->hidden);
-    if ((ln_fused & 1) && layer->o.format == ET_FMT_DENSE &&
+    const et::NarrowPlan narrow = layer->o.format == ET_FMT_DENSE
+                                      ? et::pick_narrow_ln(T, layer->hidden, layer->vdim)
+                                      : et::NarrowPlan{0, 0};
+    if (narrow.splits > 0) {
+        if ((st = et::narrow_linear_ln(narrow, b.z, layer->vdim,
+                                       reinterpret_cast<const __half*>(layer->o.weight),
+                                       reinterpret_cast<const __half*>(layer->o.bias), xin,
+                                       reinterpret_cast<const __half*>(layer->ln1_gamma),
+                                       reinterpret_cast<const __half*>(layer->ln1_beta), b.y, b.part, T,
+                                       layer->hidden, s)) != ET_OK)
+            return st;
+    } else if ((ln_fused & 1) && layer->o.format == ET_FMT_DENSE &&
         et::gemm_ln_applies(T, layer->hidden, layer->vdim)) {
         // O projection, residual and LayerNorm in one kernel
         if ((st = et::launch_gemm_ln(b.z, layer->vdim,

@@ -808,6 +808,19 @@ int pick_tall(int M, int N, int K) {
     return best_bn;
 }
 
+int g_force_narrow = -1;  // test hook: -1 = automatic, 0 = never, 32 / 64 = always that width
+
+// Width of the one-tile-per-CTA kernel for few output tiles (gemm_narrow.cu), or 0.
+int pick_narrow(int M, int N) {
+    if (g_force_narrow >= 0) return g_force_narrow;
+    if (g_force_bn != 0 || g_force_persist >= 0 || g_force_pair > 0 || g_force_tall > 0) return 0;
+    const long sms = sm_count() > 0 ? sm_count() : 148;
+    const long mt = (M + BM - 1) / BM;
+    if (mt * ((N + 31) / 32) <= sms) return 32;
+    if (mt * ((N + 63) / 64) <= sms) return 64;
+    return 0;
+}
+
 template <bool B_MN>
 int dispatch(const TilePlan& p, const CUtensorMap& tmA, const CUtensorMap& tmB,
              const CUtensorMap& tmY, const GemmArgs& args, int zdim, cudaStream_t stream) {
@@ -860,6 +873,7 @@ void gemm_force_persist(int mode) { g_force_persist = mode; }
 void gemm_set_max_ctas(int n) { g_max_ctas = n; }
 void gemm_force_pair(int mode) { g_force_pair = mode; }
 void gemm_force_tall(int mode) { g_force_tall = mode; }
+void gemm_force_narrow(int mode) { g_force_narrow = mode; }
 
 // ---- built-in gather scratch of et_linear_col_noalloc_fwd -------------------------------
 // Callers that cannot allocate device memory (see the entry point) use this array instead of
@@ -897,6 +911,9 @@ int launch_gemm_f16(const __half* X, int ldx, const __half* W, int ldw, const __
     if (!device_error_word()) return ET_ERR_NO_DEVICE;
 
     if (col_map == nullptr) {
+        const int narrow_bn = pick_narrow(M, N);
+        if (narrow_bn != 0)
+            return launch_gemm_narrow(X, ldx, W, ldw, bias, Y, ldy, M, N, K, act, narrow_bn, 1, false, stream);
         const int pair_bn = pick_pair(M, N, K);
         if (pair_bn != 0)
             return launch_gemm_pair_f16(X, ldx, W, ldw, bias, Y, ldy, M, N, K, act, pair_bn, stream);
@@ -1012,6 +1029,8 @@ void et_debug_set_gemm_max_ctas(int n) { et::gemm_set_max_ctas(n); }
 void et_debug_force_gemm_tall(int mode) { et::gemm_force_tall(mode); }
 // Test hook: -1 = automatic, 0 = single-CTA kernels only, 128 / 256 = CTA-pair tiles of that width.
 void et_debug_force_gemm_pair(int mode) { et::gemm_force_pair(mode); }
+// Test hook: -1 = automatic, 0 = never, 32 / 64 = one 128-row tile of that width per CTA.
+void et_debug_force_gemm_narrow(int mode) { et::gemm_force_narrow(mode); }
 // Test hook: -1 = automatic, 0 = one tile per CTA, 1 = persistent CTAs.
 void et_debug_force_gemm_persist(int mode) { et::gemm_force_persist(mode); }
 #endif  // ET_TEST_HOOKS

@@ -24,6 +24,13 @@ int launch_gemm_tall_f16(const __half* X, int ldx, const __half* W, int ldw, con
                          __half* Y, int ldy, int M, int N, int K, int act, int bn,
                          cudaStream_t stream);
 
+// The same product, or fp32 K-slice sums [splits][M, N] without bias (partial), on 128 x bn tiles (bn =
+// 32, 64 or, partial only, 128), one per CTA: for few output tiles; see gemm_narrow.cu.  Arguments as launch_gemm_f16's,
+// already checked.
+int launch_gemm_narrow(const __half* X, int ldx, const __half* W, int ldw, const __half* bias, void* Y,
+                       int ldy, int M, int N, int K, int act, int bn, int splits, bool partial,
+                       cudaStream_t stream);
+
 // Fused Q/K/V projection + attention for seq <= 128 and 64-wide heads; see qkv_attention.cu.
 bool qkv_attention_applies(int seq, int nhead, int kdim, int vdim);
 int launch_qkv_attention(const __half* X, const __half* Wqkv, const __half* bqkv, __half* Z,

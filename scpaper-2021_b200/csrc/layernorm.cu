@@ -127,77 +127,85 @@ skip_layernorm_kernel(const __half* __restrict__ src, const __half* __restrict__
 
 // Same normalisation fed by split-K partial sums: the row is
 //   sum_p partials[p][row, :] + bias + skip[row, :]
-// so the GEMM that precedes it never rounds its result to fp16 nor adds its bias.
-__global__ void __launch_bounds__(LN_WARPS * 32)
-skip_layernorm_partials_kernel(const float* __restrict__ partials, int nsplit, size_t split_stride,
+// so the GEMM that precedes it never rounds its result to fp16 nor adds its bias.  One CTA per row and
+// one thread per 8 columns: all of a row's loads (NS slices of 32 bytes and the residual per thread) are
+// in flight at once, so a row costs one L2 round trip and one block reduction.
+constexpr int LNP_MAX_WARPS = 8;  // rows up to 2048
+template <int NS>
+__global__ void __launch_bounds__(LNP_MAX_WARPS * 32)
+skip_layernorm_partials_kernel(const float* __restrict__ partials, size_t split_stride,
                                const __half* __restrict__ bias, const __half* __restrict__ skip,
                                const __half* __restrict__ gamma, const __half* __restrict__ beta,
-                               __half* __restrict__ out, int rows, int size, float eps) {
+                               __half* __restrict__ out, int size, float eps) {
+    __shared__ float2 s_sum[LNP_MAX_WARPS];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int row = blockIdx.x * LN_WARPS + warp;
+    const int c = threadIdx.x;  // 8-column piece
+    const bool live = c < (size >> 3);
+    const size_t at = static_cast<size_t>(blockIdx.x) * size + c * 8;
+    uint4 gq = make_uint4(0u, 0u, 0u, 0u), bq = gq, wq = gq, kq = gq;
+    if (live) {  // weights: before the wait for the kernels that produce the rest
+        gq = __ldg(reinterpret_cast<const uint4*>(gamma) + c);
+        bq = __ldg(reinterpret_cast<const uint4*>(beta) + c);
+        if (bias) wq = __ldg(reinterpret_cast<const uint4*>(bias) + c);
+    }
     pdl_launch_dependents();
     pdl_wait();
-    if (row >= rows) return;
-    const int nchunk = size >> 3;
-    const uint4* k4 =
-        skip ? reinterpret_cast<const uint4*>(skip + static_cast<size_t>(row) * size) : nullptr;
-    uint4* o4 = reinterpret_cast<uint4*>(out + static_cast<size_t>(row) * size);
-    float cache[LN_MAX_CHUNKS][8];
+    float4 p[NS][2];
+    if (live) {
+        if (skip) kq = __ldcg(reinterpret_cast<const uint4*>(skip + at));
+#pragma unroll
+        for (int i = 0; i < NS; ++i) {
+            const float4* src = reinterpret_cast<const float4*>(partials + i * split_stride + at);
+            p[i][0] = __ldcg(src);
+            p[i][1] = __ldcg(src + 1);
+        }
+    }
+    float v[8], w[8];
     float sum = 0.f, sq = 0.f;
 #pragma unroll
-    for (int it = 0; it < LN_MAX_CHUNKS; ++it) {
-        const int c = lane + it * 32;
-        if (c < nchunk) {
-            float v[8];
+    for (int j = 0; j < 8; ++j) v[j] = 0.f;
+    if (live) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = 0.f;
-            for (int p = 0; p < nsplit; ++p) {
-                const float4* src = reinterpret_cast<const float4*>(
-                    partials + p * split_stride + static_cast<size_t>(row) * size + c * 8);
-                const float4 a = __ldcg(src), b = __ldcg(src + 1);
-                v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w;
-                v[4] += b.x; v[5] += b.y; v[6] += b.z; v[7] += b.w;
-            }
-            float w[8];
-            if (bias) {
-                unpack8(__ldg(reinterpret_cast<const uint4*>(bias) + c), w);
+        for (int i = 0; i < NS; ++i) {
+            v[0] += p[i][0].x; v[1] += p[i][0].y; v[2] += p[i][0].z; v[3] += p[i][0].w;
+            v[4] += p[i][1].x; v[5] += p[i][1].y; v[6] += p[i][1].z; v[7] += p[i][1].w;
+        }
+        unpack8(wq, w);
 #pragma unroll
-                for (int j = 0; j < 8; ++j) v[j] += w[j];
-            }
-            if (k4) {
-                unpack8(__ldcg(k4 + c), w);
+        for (int j = 0; j < 8; ++j) v[j] += w[j];
+        unpack8(kq, w);
 #pragma unroll
-                for (int j = 0; j < 8; ++j) v[j] += w[j];
-            }
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                sum += v[j];
-                sq += v[j] * v[j];
-                cache[it][j] = v[j];
-            }
+        for (int j = 0; j < 8; ++j) {
+            v[j] += w[j];
+            sum += v[j];
+            sq += v[j] * v[j];
         }
     }
     sum = warp_sum(sum);
     sq = warp_sum(sq);
+    if (lane == 0) s_sum[warp] = make_float2(sum, sq);
+    __syncthreads();
+    sum = 0.f;
+    sq = 0.f;
+    for (int i = 0; i < static_cast<int>(blockDim.x >> 5); ++i) {
+        sum += s_sum[i].x;
+        sq += s_sum[i].y;
+    }
     const float mean = sum / size;
     const float var = fmaxf(sq / size - mean * mean, 0.f);
     const float rstd = rsqrtf(var + eps);
+    if (live) {
+        float g[8], b[8];
+        unpack8(gq, g);
+        unpack8(bq, b);
 #pragma unroll
-    for (int it = 0; it < LN_MAX_CHUNKS; ++it) {
-        const int c = lane + it * 32;
-        if (c < nchunk) {
-            float g[8], b[8], v[8];
-            unpack8(__ldg(reinterpret_cast<const uint4*>(gamma) + c), g);
-            unpack8(__ldg(reinterpret_cast<const uint4*>(beta) + c), b);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = (cache[it][j] - mean) * rstd * g[j] + b[j];
-            uint4 o;
-            o.x = pack_half2(v[0], v[1]);
-            o.y = pack_half2(v[2], v[3]);
-            o.z = pack_half2(v[4], v[5]);
-            o.w = pack_half2(v[6], v[7]);
-            o4[c] = o;
-        }
+        for (int j = 0; j < 8; ++j) v[j] = (v[j] - mean) * rstd * g[j] + b[j];
+        uint4 o;
+        o.x = pack_half2(v[0], v[1]);
+        o.y = pack_half2(v[2], v[3]);
+        o.z = pack_half2(v[4], v[5]);
+        o.w = pack_half2(v[6], v[7]);
+        *reinterpret_cast<uint4*>(out + at) = o;
     }
 }
 
@@ -281,13 +289,17 @@ int launch_skip_layernorm_partials(const float* partials, int nsplit, size_t spl
                                    cudaStream_t stream) {
     if (!partials || !gamma || !beta || !out || rows <= 0 || size <= 0 || nsplit <= 0)
         return ET_ERR_INVALID_ARG;
-    if (size % 8 || size > LN_MAX_CHUNKS * 8 * 32) return ET_ERR_SHAPE;
-    const int blocks = (rows + LN_WARPS - 1) / LN_WARPS;
-    return launch_kernel(skip_layernorm_partials_kernel, dim3(blocks), dim3(LN_WARPS * 32), 0,
-                         stream, partials, nsplit, split_stride, bias, skip, gamma, beta, out, rows,
-                         size, 1e-5f) == cudaSuccess
-               ? ET_OK
-               : ET_ERR_CUDA;
+    if (size % 8 || size > LNP_MAX_WARPS * 32 * 8 || nsplit > 4) return ET_ERR_SHAPE;
+    const int threads = (size / 8 + 31) / 32 * 32;
+    auto go = [&](auto kern) {
+        return launch_kernel(kern, dim3(rows), dim3(threads), 0, stream, partials, split_stride, bias, skip,
+                             gamma, beta, out, size, 1e-5f);
+    };
+    const cudaError_t e = nsplit == 1   ? go(skip_layernorm_partials_kernel<1>)
+                          : nsplit == 2 ? go(skip_layernorm_partials_kernel<2>)
+                          : nsplit == 3 ? go(skip_layernorm_partials_kernel<3>)
+                                        : go(skip_layernorm_partials_kernel<4>);
+    return e == cudaSuccess ? ET_OK : ET_ERR_CUDA;
 }
 
 }  // namespace et

@@ -13,8 +13,10 @@
 // two-stage ring (2 x 40 KB) that is reused, once the projection's products are complete, for
 // the Q, K, V tiles (3 x 16 KB) and the probability tile (32 KB, later the output staging
 // tile); 256 tensor-memory columns: Q | K | V accumulators in [0, 192), then S in [0, 128) and
-// O in [192, 256).  Two CTAs fit one SM.  All waits are bounded.
+// O in [192, 256).  All waits are bounded.
 #include <math.h>
+
+#include <type_traits>
 
 #include "common.cuh"
 #include "gemm_common.cuh"
@@ -39,13 +41,13 @@ constexpr int QA_THREADS = 320;
 constexpr int QA_SM_THREADS = 256;
 constexpr int QA_ATOM = 128 * 128;               // 128 rows x 64 fp16
 constexpr int QA_STAGE = QA_ATOM + 3 * 64 * 128; // X block + three weight slices = 40 KB
-constexpr int QA_STAGES = 2;
-constexpr int QA_RING = QA_STAGES * QA_STAGE;    // 80 KB = Q + K + V + 2 atoms of P
 constexpr int QA_MISC = 256 + 192 * 4 + 6 * 128 * 4;
-constexpr int QA_SMEM = QA_RING + QA_MISC + 1024;
+constexpr int QA_MAX_STAGES = 5;
+__host__ __device__ constexpr int qa_smem(int stages) { return stages * QA_STAGE + QA_MISC + 1024; }
 constexpr int QA_TMEM = 256;
-static_assert(QA_RING == 5 * QA_ATOM, "ring must hold Q, K, V and two atoms of P");
-static_assert(QA_SMEM <= 113 * 1024, "two CTAs per SM");
+static_assert(2 * QA_STAGE == 5 * QA_ATOM, "two stages must hold Q, K, V and two atoms of P");
+static_assert(qa_smem(2) <= 113 * 1024, "two CTAs per SM");
+static_assert(qa_smem(QA_MAX_STAGES) <= 227 * 1024, "shared memory budget exceeded");
 
 struct QkvAttnArgs {
     const __half* bias;  // [2 * kdim + vdim] or null
@@ -59,8 +61,8 @@ struct QkvAttnArgs {
 
 // MASK: the mask kind, compiled in (run-time branches around the softmax code cost issue
 // efficiency, as they did in the GEMM epilogues).
-template <int MASK>
-__global__ void __launch_bounds__(QA_THREADS, 2)
+template <int MASK, int QA_STAGES>
+__global__ void __launch_bounds__(QA_THREADS, (QA_STAGES == 2 ? 2 : 1))
 qkv_attention_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW,
                      const __grid_constant__ CUtensorMap tmZ, const QkvAttnArgs a) {
     extern __shared__ uint8_t smem_raw[];
@@ -69,15 +71,15 @@ qkv_attention_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
     uint8_t* sK = smem + QA_ATOM;
     uint8_t* sV = smem + 2 * QA_ATOM;
     uint8_t* sP = smem + 3 * QA_ATOM;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + QA_RING);
-    uint64_t* full_bar = bars;       // [2]
-    uint64_t* empty_bar = bars + 2;  // [2]
-    uint64_t* proj_full = bars + 4;
-    uint64_t* qkv_ready = bars + 5;
-    uint64_t* s_full = bars + 6;
-    uint64_t* p_full = bars + 7;
-    uint64_t* o_full = bars + 8;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 9);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + QA_STAGES * QA_STAGE);
+    uint64_t* full_bar = bars;                       // [QA_STAGES]
+    uint64_t* empty_bar = full_bar + QA_MAX_STAGES;  // [QA_STAGES]
+    uint64_t* proj_full = empty_bar + QA_MAX_STAGES;
+    uint64_t* qkv_ready = proj_full + 1;
+    uint64_t* s_full = proj_full + 2;
+    uint64_t* p_full = proj_full + 3;
+    uint64_t* o_full = proj_full + 4;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(proj_full + 5);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     float* s_bias = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + 256);  // [192]
     float* s_x = s_bias + 192;  // max exchange [2][128], sum exchange [2][128]
@@ -459,18 +461,23 @@ int launch_qkv_attention(const __half* X, const __half* Wqkv, const __half* bqkv
     }
     int dev = 0;
     cudaGetDevice(&dev);
-    auto go = [&](auto kern, int slot, const QkvAttnArgs& args) -> int {
-        static std::atomic<bool> attr_set[4][64] = {};
+    auto go = [&](auto kern, int slot, int smem, const QkvAttnArgs& args) -> int {
+        static std::atomic<bool> attr_set[8][64] = {};
         if (dev >= 0 && dev < 64 && !attr_set[slot][dev]) {
-            if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, QA_SMEM) !=
-                cudaSuccess)
+            if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
                 return ET_ERR_CUDA;
             attr_set[slot][dev] = true;
         }
-        return launch_kernel(kern, dim3(nhead, batch), dim3(QA_THREADS), QA_SMEM, stream, tmX, tmW,
-                             tmZ, args) == cudaSuccess
+        return launch_kernel(kern, dim3(nhead, batch), dim3(QA_THREADS), smem, stream, tmX, tmW, tmZ,
+                             args) == cudaSuccess
                    ? ET_OK
                    : ET_ERR_CUDA;
+    };
+    const bool deep = static_cast<long>(nhead) * batch <= sm_count();
+    auto by_depth = [&](auto mask, const QkvAttnArgs& args) -> int {
+        constexpr int M = decltype(mask)::value;
+        return deep ? go(qkv_attention_kernel<M, QA_MAX_STAGES>, 4 + M, qa_smem(QA_MAX_STAGES), args)
+                    : go(qkv_attention_kernel<M, 2>, M, qa_smem(2), args);
     };
     QkvAttnArgs a;
     a.bias = bqkv;
@@ -483,10 +490,10 @@ int launch_qkv_attention(const __half* X, const __half* Wqkv, const __half* bqkv
     a.scale_log2 = scale * 1.4426950408889634f;
     a.err_word = err;
     switch (mask_kind) {
-        case ET_MASK_CAUSAL: return go(qkv_attention_kernel<ET_MASK_CAUSAL>, 1, a);
-        case ET_MASK_PADDING: return go(qkv_attention_kernel<ET_MASK_PADDING>, 2, a);
-        case ET_MASK_ADDITIVE: return go(qkv_attention_kernel<ET_MASK_ADDITIVE>, 3, a);
-        default: return go(qkv_attention_kernel<ET_MASK_NONE>, 0, a);
+        case ET_MASK_CAUSAL: return by_depth(std::integral_constant<int, ET_MASK_CAUSAL>{}, a);
+        case ET_MASK_PADDING: return by_depth(std::integral_constant<int, ET_MASK_PADDING>{}, a);
+        case ET_MASK_ADDITIVE: return by_depth(std::integral_constant<int, ET_MASK_ADDITIVE>{}, a);
+        default: return by_depth(std::integral_constant<int, ET_MASK_NONE>{}, a);
     }
 }
 
