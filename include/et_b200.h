@@ -414,24 +414,6 @@ int et_encoder_layer_fwd(const et_encoder_layer_t* layer, const et_half* x, et_h
                          const int32_t* valid_len, void* workspace, size_t workspace_bytes,
                          et_stream stream);
 
-/* A stack of layers as one call: layer i reads the previous layer's output (layer 0: x) and writes
- * buf0 (even i) or buf1 (odd i), each [batch * seq, hidden] and, like the workspace, the caller's for the
- * life of the stack.  _create copies the descriptions.  _fwd issues every layer's kernels on `stream`;
- * when a call repeats the arguments of an earlier one it replays that call's launches as one CUDA
- * graph (kernels read their operands at every replay; up to 8 argument sets are recorded, and none on
- * a stream that is being captured).  `layers`, if given, are the current descriptions: a change since
- * _create drops the recorded launches.  Unlike the other entry points _create and _fwd may allocate
- * (host memory, graph objects).  Calls on one stack are serialised; as they share its buffers, two of
- * them must not overlap on the GPU either.  _destroy only after the stack's work has completed.
- * Stands in for the reference's loop over Encoder objects (test/Table2/template.hpp). */
-typedef struct et_encoder_stack et_encoder_stack_t;
-int et_encoder_stack_create(const et_encoder_layer_t* const* layers, int n_layers, int batch, int seq,
-                            et_half* buf0, et_half* buf1, void* workspace, size_t workspace_bytes,
-                            et_encoder_stack_t** stack);
-int et_encoder_stack_fwd(et_encoder_stack_t* stack, const et_encoder_layer_t* const* layers, const et_half* x,
-                         int mask_kind, const et_half* mask, const int32_t* valid_len, et_stream stream);
-int et_encoder_stack_destroy(et_encoder_stack_t* stack);
-
 /* =================================================================================
  * Head-parallel form of the layer, for ONE long sequence spread over several GPUs (the
  * reference is single-GPU; this is the tensor-parallel reading of Attention/Attention.h:

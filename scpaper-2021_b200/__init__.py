@@ -39,7 +39,6 @@ ABI_SYMBOLS = [
     "et_attention_fuse_o_fwd", "et_attention_fuse_o_single_launch_fwd",
     "et_fused_vo_attention_fwd", "et_linear_vo_fwd",
     "et_encoder_layer_workspace_bytes", "et_encoder_layer_fwd",
-    "et_encoder_stack_create", "et_encoder_stack_fwd", "et_encoder_stack_destroy",
     "et_attention_units_fwd", "et_encoder_attention_units_fwd", "et_encoder_after_attention_fwd",
 ]
 
@@ -160,7 +159,6 @@ _SIGNATURES = {
     "et_fused_vo_attention_fwd": "ppppp" "iiiiiiii" "ppfp",
     "et_fused_vo_attention_pruned_fwd": "ppppippp" "iiiiiiii" "ppfp",
     "et_encoder_layer_fwd": "pppiii" "pppzp",
-    "et_encoder_stack_fwd": "pppi" "ppp",
 }
 _KINDS = {"p": c_void_p, "i": c_int, "z": c_size_t, "f": c_float}
 _calls = {}
@@ -928,8 +926,7 @@ class PeerExchange:
 
 
 class EncoderStack:
-    """N chained encoder layers, issued as one native call (et_encoder_stack_fwd: repeated calls are
-    replayed as a CUDA graph).  The batch can be cut into `lanes` groups of sequences that
+    """N chained encoder layers.  The batch can be cut into `lanes` groups of sequences that
     run through the whole stack on streams of their own (sequences are independent), so that
     the kernels of one group fill the SMs another group's kernels leave idle; each group has
     its own workspace, all share two ping-pong activation buffers."""
@@ -956,36 +953,8 @@ class EncoderStack:
         self.workspace = self.workspaces[0]
         self.buf = [torch.empty((batch * seq, hidden), dtype=torch.float16, device=device)
                     for _ in range(2)]
-        self._native = None  # (layers, descriptions, native handle) of the one-lane form
         self.streams = [torch.cuda.Stream(device=device) for _ in self.groups[1:]]
         self.events = [(torch.cuda.Event(), torch.cuda.Event()) for _ in self.groups[1:]]
-
-    def _native_stack(self):
-        if self._native is None or self._native[0] != self.layers:
-            self.close()
-            descs = (c_void_p * len(self.layers))(*[ctypes.addressof(l.desc) for l in self.layers])
-            handle = c_void_p(None)
-            ws = self.workspace
-            check(lib().et_encoder_stack_create(descs, c_int(len(self.layers)), c_int(self.batch),
-                                                c_int(self.seq), _p(self.buf[0]), _p(self.buf[1]), _p(ws),
-                                                c_size_t(ws.numel() * ws.element_size()),
-                                                ctypes.byref(handle)), "et_encoder_stack_create")
-            self._native = (list(self.layers), descs, handle)
-        return self._native
-
-    def close(self) -> None:
-        """Gives the native plan back (its recorded launches; the buffers are this object's)."""
-        native, self._native = getattr(self, "_native", None), None
-        if native is not None and _lib is not None:
-            import torch
-            torch.cuda.synchronize(self.buf[0].device)
-            _lib.et_encoder_stack_destroy(native[2])
-
-    def __del__(self):
-        try:
-            self.close()
-        except Exception:  # noqa: BLE001 - interpreter shutdown
-            pass
 
     def _run_group(self, g, x, mask_kind, mask, valid_len):
         first, n = self.groups[g]
@@ -998,11 +967,6 @@ class EncoderStack:
             cur = out
 
     def forward(self, x, mask_kind=MASK_NONE, mask=None, valid_len=None):
-        if len(self.groups) == 1:
-            native = self._native_stack()
-            _call("et_encoder_stack_fwd", native[2], native[1], _a(x), mask_kind, _a(mask), _a(valid_len),
-                  _raw_stream())
-            return self.buf[(len(self.layers) - 1) & 1]
         import torch
         main = torch.cuda.current_stream()
         for g in range(1, len(self.groups)):

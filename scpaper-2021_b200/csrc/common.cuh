@@ -68,7 +68,6 @@ enum : int {
 // Every kernel launch of the library is counted on the host (et_launch_count), so that a
 // caller can state how many kernels one call issued.
 void count_launch();
-void count_launches(long long n);
 
 // Launches `kernel` with the programmatic-stream-serialization attribute when PDL is on.
 template <typename... KArgs, typename... Args>

@@ -55,7 +55,6 @@ bool g_pdl = true;
 }
 bool pdl_enabled() { return g_pdl; }
 void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
-void count_launches(long long n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 void set_pdl_enabled(bool on) { g_pdl = on; }
 
 int* device_error_word() {
