@@ -52,9 +52,11 @@ int g_ln_fusion = -1;
 // FFN2, +10 % on the whole stack); with several waves the wider tiles and CTA pairs of the plain
 // GEMM win by more than the LayerNorm launch costs (8192 tokens: -3 %).  A cluster must fit one
 // GPC, so the number of resident clusters comes from the occupancy query, not from the SM count.
-int ln_fusion_mask(int T, int hidden) {
-    if (g_ln_fusion >= 0) return g_ln_fusion;
-    return et_linear_skip_layernorm_pays(T, hidden, hidden) ? 3 : 0;
+// With many rows the same fusion runs on persistent clusters of CTA pairs (gemm_pair_ln.cu), where
+// it depends on K as well.
+bool ln_fused(int bit, int T, int hidden, int K) {
+    if (g_ln_fusion >= 0) return (g_ln_fusion & bit) != 0;
+    return et_linear_skip_layernorm_pays(T, K, hidden) != 0;
 }
 
 // How a dense [T, K] x [hidden, K]^T product followed by residual + LayerNorm runs with few row blocks:
@@ -213,7 +215,6 @@ int ffn_block(const et_encoder_layer_t* layer, const LayerBuffers& b, int T, __h
               cudaStream_t s) {
     int st;
     et_half* out = reinterpret_cast<et_half*>(out_h);
-    const int ln_fused = ln_fusion_mask(T, layer->hidden);
     // ffn2 as the dense product it amounts to: W2 itself, or - for the compressed pair - the
     // kept columns of W2 on the kept hidden units
     const __half* w2 = reinterpret_cast<const __half*>(layer->ffn2.weight);
@@ -239,7 +240,7 @@ int ffn_block(const et_encoder_layer_t* layer, const LayerBuffers& b, int T, __h
                                 reinterpret_cast<const __half*>(layer->ln2_gamma),
                                 reinterpret_cast<const __half*>(layer->ln2_beta), out_h, b.part, T,
                                 layer->hidden, s);
-    if ((ln_fused & 2) && ffn2_dense && gemm_ln_applies(T, layer->hidden, k2) &&
+    if (ffn2_dense && ln_fused(2, T, layer->hidden, k2) && gemm_ln_applies(T, layer->hidden, k2) &&
         reinterpret_cast<const __half*>(out) != b.y) {
         // FFN2, residual and LayerNorm in one kernel
         return launch_gemm_ln(b.f, k2, w2, k2,
@@ -357,7 +358,6 @@ int et_encoder_layer_fwd(const et_encoder_layer_t* layer, const et_half* x, et_h
             ET_OK)
             return st;
     }
-    const int ln_fused = et::ln_fusion_mask(T, layer->hidden);
     const et::NarrowPlan narrow = layer->o.format == ET_FMT_DENSE
                                       ? et::pick_narrow_ln(T, layer->hidden, layer->vdim)
                                       : et::NarrowPlan{0, 0};
@@ -369,8 +369,8 @@ int et_encoder_layer_fwd(const et_encoder_layer_t* layer, const et_half* x, et_h
                                        reinterpret_cast<const __half*>(layer->ln1_beta), b.y, b.part, T,
                                        layer->hidden, s)) != ET_OK)
             return st;
-    } else if ((ln_fused & 1) && layer->o.format == ET_FMT_DENSE &&
-        et::gemm_ln_applies(T, layer->hidden, layer->vdim)) {
+    } else if (layer->o.format == ET_FMT_DENSE && et::ln_fused(1, T, layer->hidden, layer->vdim) &&
+               et::gemm_ln_applies(T, layer->hidden, layer->vdim)) {
         // O projection, residual and LayerNorm in one kernel
         if ((st = et::launch_gemm_ln(b.z, layer->vdim,
                                      reinterpret_cast<const __half*>(layer->o.weight), layer->vdim,

@@ -123,6 +123,15 @@ int launch_gemm_ln(const __half* X, int ldx, const __half* W, int ldw, const __h
                    const __half* resid, int ldr, const __half* gamma, const __half* beta,
                    __half* out, int ldo, int M, int N, int K, cudaStream_t stream);
 
+// The same on persistent clusters of CTA pairs, for many rows (gemm_pair_ln.cu; N = 512, 768 or 1024).
+// _pays: whether it is expected to beat the plain GEMM and a LayerNorm pass.  resid not null; arguments
+// already checked.
+bool gemm_pair_ln_applies(int M, int N, int K);
+bool gemm_pair_ln_pays(int M, int N, int K);
+int launch_gemm_pair_ln(const __half* X, int ldx, const __half* W, int ldw, const __half* bias,
+                        const __half* resid, int ldr, const __half* gamma, const __half* beta, __half* out,
+                        int ldo, int M, int N, int K, cudaStream_t stream);
+
 // out = LN(src + skip) * gamma + beta (skip may be null).
 int launch_skip_layernorm(const __half* src, const __half* skip, const __half* gamma,
                           const __half* beta, __half* out, int rows, int size,
