@@ -564,6 +564,44 @@ __device__ __forceinline__ float gelu_tanh(float x) {
     return x * (0.5f + 0.5f * t);
 }
 
+// Two fp32 numbers in one 64-bit register, added and multiplied by one instruction (each lane rounds
+// as the scalar instruction does).
+__device__ __forceinline__ uint64_t pack_f32x2(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack_f32x2(uint64_t v, float& a, float& b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// gelu_tanh of both lanes: the same operations in the same order.
+__device__ __forceinline__ uint64_t gelu_tanh_f32x2(uint64_t x) {
+    const uint64_t c1 = pack_f32x2(0.035677408136300125f, 0.035677408136300125f);
+    const uint64_t c0 = pack_f32x2(0.7978845608028654f, 0.7978845608028654f);
+    const uint64_t half = pack_f32x2(0.5f, 0.5f);
+    float u0, u1;
+    unpack_f32x2(mul_f32x2(x, fma_f32x2(mul_f32x2(c1, x), x, c0)), u0, u1);
+    asm("tanh.approx.f32 %0, %0;" : "+f"(u0));
+    asm("tanh.approx.f32 %0, %0;" : "+f"(u1));
+    return mul_f32x2(x, fma_f32x2(half, pack_f32x2(u0, u1), half));
+}
+
 __device__ __forceinline__ float apply_act(float x, int act) {
     if (act == ET_ACT_RELU) return fmaxf(x, 0.f);
     if (act == ET_ACT_GELU) return gelu_tanh(x);

@@ -48,17 +48,20 @@ __device__ __forceinline__ void stage_f16_chunk(const uint32_t (&r)[32], const f
     for (int gq = 0; gq < 4; ++gq) {
         const float4 b0 = *reinterpret_cast<const float4*>(bias32 + gq * 8);
         const float4 b1 = *reinterpret_cast<const float4*>(bias32 + gq * 8 + 4);
+        const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
         float v[8];
-        v[0] = __uint_as_float(r[gq * 8 + 0]) + b0.x;
-        v[1] = __uint_as_float(r[gq * 8 + 1]) + b0.y;
-        v[2] = __uint_as_float(r[gq * 8 + 2]) + b0.z;
-        v[3] = __uint_as_float(r[gq * 8 + 3]) + b0.w;
-        v[4] = __uint_as_float(r[gq * 8 + 4]) + b1.x;
-        v[5] = __uint_as_float(r[gq * 8 + 5]) + b1.y;
-        v[6] = __uint_as_float(r[gq * 8 + 6]) + b1.z;
-        v[7] = __uint_as_float(r[gq * 8 + 7]) + b1.w;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = act_fn<ACT>(v[j]);
+        for (int j = 0; j < 8; j += 2) {
+            uint64_t x = add_f32x2(
+                pack_f32x2(__uint_as_float(r[gq * 8 + j]), __uint_as_float(r[gq * 8 + j + 1])),
+                pack_f32x2(b[j], b[j + 1]));
+            if (ACT == ET_ACT_GELU) x = gelu_tanh_f32x2(x);
+            unpack_f32x2(x, v[j], v[j + 1]);
+            if (ACT == ET_ACT_RELU) {
+                v[j] = fmaxf(v[j], 0.f);
+                v[j + 1] = fmaxf(v[j + 1], 0.f);
+            }
+        }
         uint4 o;
         o.x = pack_half2(v[0], v[1]);
         o.y = pack_half2(v[2], v[3]);
