@@ -44,12 +44,15 @@ attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     attention_cta<MASK, false>(tmQ, tmK, tmV, tmZ, a, smem, q0, h, blockIdx.z, 0u, nullptr);
 }
 
+bool g_attention_rows = true;  // test hook: false = always the two-threads-per-row kernel
+
 int launch_attention_impl(const __half* Q, const __half* K, const __half* V, __half* Z, int batch,
                           int seq, int nhead, int dh_qk, int dh_v, int ldq, int ldk, int ldv,
                           int ldz, int mask_kind, const __half* mask, const int* valid_len,
                           float scale, const int* col_id, const int* head_ptr, int nnz_col,
                           cudaStream_t stream, const int* unit_head = nullptr,
-                          const int* unit_first = nullptr, int n_units = 0, int blocks_per_unit = 0) {
+                          const int* unit_first = nullptr, int n_units = 0, int blocks_per_unit = 0,
+                          bool row_per_thread = true) {
     if (n_units < 0 || n_units > ATT_MAX_UNITS) return ET_ERR_SHAPE;
     if (n_units > 0) {
         if (!unit_head || !unit_first || blocks_per_unit <= 0) return ET_ERR_INVALID_ARG;
@@ -124,6 +127,14 @@ int launch_attention_impl(const __half* Q, const __half* K, const __half* V, __h
     }
     const dim3 grid = n_units > 0 ? dim3(blocks_per_unit, n_units, batch)
                                   : dim3((seq + BQ - 1) / BQ, nhead, batch);
+    // Heads of up to 64 features: one query row per thread, probabilities in tensor memory
+    // (attention_rows.cu; figures there).  Wider heads do not leave room for P beside S and O in half an
+    // SM's tensor memory, a compressed V needs the scattering epilogue, and an additive mask is bound by its
+    // own loads, which half-rows spread over twice the warps (16 x 128, 12 heads: 41 against 43 us): they
+    // take the kernel below.
+    if (!pruned && mask_kind != ET_MASK_ADDITIVE && row_per_thread && g_attention_rows &&
+        attention_rows_applies(dh_qk, dh_v, grid))
+        return launch_attention_rows(tmQ, tmK, tmV, tmZ, a, grid, stream);
     auto go = [&](auto kern, int slot) -> int {
         static std::atomic<bool> attr_set[4][64] = {};
         if (dev >= 0 && dev < 64 && !attr_set[slot][dev]) {
@@ -150,9 +161,10 @@ int launch_attention_impl(const __half* Q, const __half* K, const __half* V, __h
 int launch_attention(const __half* Q, const __half* K, const __half* V, __half* Z, int batch,
                      int seq, int nhead, int dh_qk, int dh_v, int ldq, int ldk, int ldv, int ldz,
                      int mask_kind, const __half* mask, const int* valid_len, float scale,
-                     cudaStream_t stream) {
+                     cudaStream_t stream, bool row_per_thread) {
     return launch_attention_impl(Q, K, V, Z, batch, seq, nhead, dh_qk, dh_v, ldq, ldk, ldv, ldz,
-                                 mask_kind, mask, valid_len, scale, nullptr, nullptr, 0, stream);
+                                 mask_kind, mask, valid_len, scale, nullptr, nullptr, 0, stream,
+                                 nullptr, nullptr, 0, 0, row_per_thread);
 }
 
 int launch_attention_units(const __half* Q, const __half* K, const __half* V, __half* Z, int batch,
@@ -169,6 +181,11 @@ int launch_attention_units(const __half* Q, const __half* K, const __half* V, __
 }  // namespace et
 
 extern "C" {
+
+#ifdef ET_TEST_HOOKS
+// Test hook: 0 = every head width on the kernel that splits a query row over two threads.
+void et_debug_set_attention_rows(int on) { et::g_attention_rows = on != 0; }
+#endif  // ET_TEST_HOOKS
 
 int et_attention_units_fwd(const et_half* Q, const et_half* K, const et_half* V, et_half* Z, int batch,
                            int seq, int nhead, int dh_qk, int dh_v, int ldq, int ldk, int ldv,

@@ -105,6 +105,12 @@ struct AttnArgs {
     unsigned short unit_first[ATT_MAX_UNITS];
 };
 
+// One query row per thread, heads of up to 64 features, dense V (attention_rows.cu).  blocks: query
+// blocks (per unit) x heads or units x sequences.
+bool attention_rows_applies(int dh_qk, int dh_v, dim3 blocks);
+int launch_attention_rows(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV,
+                          const CUtensorMap& tmZ, const AttnArgs& a, dim3 blocks, cudaStream_t stream);
+
 // The work of one CTA: queries [q0, q0 + 128) of head h of sequence b.  `smem` is the CTA's
 // 1024-byte-aligned dynamic shared memory.
 // MASK: the mask kind, compiled in (keeps the mask bookkeeping out of the registers of the

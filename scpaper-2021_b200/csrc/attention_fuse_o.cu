@@ -262,7 +262,7 @@ int launch_attention_fuse_o(const __half* Q, const __half* K, const __half* V, c
                        vdim_l <= MAX_IN;
     if (!fused) {
         int st = launch_attention(Q, K, V, Z, batch, seq, nhead, dh_qk, dh_v, ldq, ldk, ldv,
-                                  static_cast<int>(vdim_l), mask_kind, mask, valid_len, scale, stream);
+                                  static_cast<int>(vdim_l), mask_kind, mask, valid_len, scale, stream, false);
         if (st != ET_OK) return st;
         return launch_linear_tile(o_row_ptr, o_row_off, o_tiles, o_nnz, o_bias, Z, out, batch * seq,
                                   static_cast<int>(vdim_l), emdim, ET_ACT_NONE, stream);

@@ -90,11 +90,12 @@ int launch_linear_expand_packed(const uint32_t* pk_mask, const int* pk_off, cons
                                 const __half* bias, const __half* X, __half* Y, int T, int in, int out,
                                 int act, cudaStream_t stream);
 
-// Fused attention (see attention.cu).  Vc_col_id / head_ptr are null for an uncompressed V.
+// Fused attention (see attention.cu).  row_per_thread = false keeps every head width on the kernel whose
+// body attention_fuse_o.cu shares, so that the two give the same bits.
 int launch_attention(const __half* Q, const __half* K, const __half* V, __half* Z, int batch,
                      int seq, int nhead, int dh_qk, int dh_v, int ldq, int ldk, int ldv, int ldz,
                      int mask_kind, const __half* mask, const int* valid_len, float scale,
-                     cudaStream_t stream);
+                     cudaStream_t stream, bool row_per_thread = true);
 
 // The same kernel over a list of work units (head, first 128-query block), each covering
 // blocks_per_unit query blocks; query rows outside the units are not written.  unit_head and
