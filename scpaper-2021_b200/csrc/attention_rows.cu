@@ -13,11 +13,13 @@
 // What bounds it: the special-function unit (16 exp2 per clock and SM: 1024 cycles a 128 x 128 block)
 // and what a warp cannot hide of its own chain: clock stamps gave 2330 cycles a block to a CTA alone and
 // 2740 to each of two, of which 300 are the maximum, 240 the raise decision and 1600 the exponentials,
-// before these drained once instead of four times a block.
+// before these drained once instead of four times a block.  Every fourth pair of exponentials runs on the
+// FMA pipe, whose issue slots are two thirds free: 1 x 4096 94.4 -> 86.9 us, 256 x 512 328 -> 309 us; 5 / 16,
+// 3 / 8 and half of them measured 88.8, 92 and 99 us on the first.
 // Against the kernel that splits a row over two threads (attention_body.cuh), 64-wide heads: 256 x 512
-// tokens, 12 heads 430 -> 328 us; 32 x 384, 16 heads 53.1 -> 39.8 us (padded 55.4 -> 45.9); 4 x 2048
-// causal, 16 heads 90 -> 62 us; 1 x 4096 98.5 -> 94.4 us (384 items on 296 CTAs: the second round is a third
-// full); 16 x 128, one item per CTA, 6.9 -> 7.0 us.
+// tokens, 12 heads 430 -> 309 us; 32 x 384, 16 heads 53 -> 38.5 us; 4 x 2048 causal, 16 heads 92 -> 60 us;
+// 1 x 4096 98.5 -> 86.9 us (384 items on 296 CTAs: the second round is a third full); 16 x 128, one item per
+// CTA, 6.9 -> 7.2 us.
 //
 // Tensor memory: S in columns [0, 128), O in [128, 192), P in [192, 256): 256 columns, two CTAs' worth.
 // All waits are bounded.
@@ -56,6 +58,33 @@ struct RowsSched {
     int items, nqb, nh, batch;
     int heavy_first;  // 1: query blocks vary slowest, the last (causal: longest) ones first
 };
+
+// 2^x of both lanes on the FMA pipe, for x <= 64: x = n + r with n whole and |r| <= 1/2, 2^r by a degree-5
+// polynomial (Remez fit of the relative error on [-1/2, 1/2]; 2.1e-7 at worst in fp32, as far off as
+// ex2.approx may be), 2^n through the exponent field.  Below -126 it returns 2^-126, which is zero as an fp16
+// probability; NaN stays NaN.
+__device__ __forceinline__ uint64_t exp2_poly_f32x2(uint64_t x2) {
+    float x0, x1;
+    unpack_f32x2(x2, x0, x1);
+    asm("max.NaN.f32 %0, %0, 0fC2FC0000;" : "+f"(x0));  // -126
+    asm("max.NaN.f32 %0, %0, 0fC2FC0000;" : "+f"(x1));
+    const uint64_t x = pack_f32x2(x0, x1);
+    const uint64_t magic = pack_f32x2(12582912.f, 12582912.f), unmagic = pack_f32x2(-12582912.f, -12582912.f);
+    const uint64_t t = add_f32x2(x, magic);  // the whole part in the low mantissa bits
+    const uint64_t minus1 = pack_f32x2(-1.f, -1.f);
+    const uint64_t r = fma_f32x2(add_f32x2(t, unmagic), minus1, x);
+    auto both = [](float c) { return pack_f32x2(c, c); };
+    uint64_t p = fma_f32x2(both(0.0013276472f), r, both(0.009675541f));
+    p = fma_f32x2(p, r, both(0.05550713f));
+    p = fma_f32x2(p, r, both(0.2402212f));
+    p = fma_f32x2(p, r, both(0.69314694f));
+    p = fma_f32x2(p, r, both(1.0000001f));
+    float t0, t1;
+    unpack_f32x2(t, t0, t1);
+    const float s0 = __uint_as_float((__float_as_uint(t0) << 23) + 0x3f800000u);
+    const float s1 = __uint_as_float((__float_as_uint(t1) << 23) + 0x3f800000u);
+    return mul_f32x2(p, pack_f32x2(s0, s1));
+}
 
 template <int MASK>
 __global__ void __launch_bounds__(AR_THREADS, 2)
@@ -358,11 +387,17 @@ attention_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
                     uint32_t p[16];
 #pragma unroll
                     for (int i = 0; i < 16; ++i) {
-                        float x0, x1;
-                        unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])),
-                                               scale2, neg_m2),
-                                     x0, x1);
-                        const float e0 = exp2_approx(x0), e1 = exp2_approx(x1);
+                        const uint64_t x2 =
+                            fma_f32x2(pack_f32x2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])),
+                                      scale2, neg_m2);
+                        float e0, e1;
+                        if ((i & 3) == 3) {
+                            unpack_f32x2(exp2_poly_f32x2(x2), e0, e1);
+                        } else {
+                            unpack_f32x2(x2, e0, e1);
+                            e0 = exp2_approx(e0);
+                            e1 = exp2_approx(e1);
+                        }
                         sum2[i & 1] = add_f32x2(sum2[i & 1], pack_f32x2(e0, e1));
                         p[i] = pack_half2(e0, e1);
                     }
