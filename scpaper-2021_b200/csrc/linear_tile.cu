@@ -119,6 +119,18 @@ int launch_tile_common(bool packed, const int* row_ptr, const int* row_off, cons
                    : ET_ERR_CUDA;
     }
 
+    // Packed weights with a long K and few output tiles: expanding the tiles into dense operands
+    // (linear_expand.cu) costs the tensor core 240 cycles a K block whatever is stored, and its narrow panels
+    // fill more SMs; this kernel's N = 16 products cost 60 each in one serial chain per 128 x 128 tile.  Measured on
+    // B200 at 80 / 90 / 95 % sparsity, this kernel against that: 3072 -> 768 at 1000 tokens (48 tiles) 18.4 / 16.5 /
+    // 14.1 against 13.8 / 13.7 / 13.5 us, 4096 -> 1024 at 1000 (64 tiles) 24.6 / 21.0 / 18.7 against 17.0 us, 2048 -> 512
+    // at 2048 (64 tiles) 14.0 / 12.7 / 11.1 against 10.3 us; with 96 tiles (3072 -> 768 at 2048) 19.7 / 17.4 / 14.9
+    // against 17.9 / 17.0 / 16.6 us, and 768-wide K gains nothing.
+    const long out_tiles = static_cast<long>((out + TBN - 1) / TBN) * ((T + TBM - 1) / TBM);
+    if (packed && (tile_packed_mode() == 2 || (tile_packed_mode() < 0 && g_tile_wide < 0 && in >= 2048 &&
+                                               2 * out_tiles <= (sm_count() > 0 ? sm_count() : 148))))
+        return launch_linear_expand_packed(pk_mask, pk_off, tiles, bias, X, Y, T, in, out, act, stream);
+
     CUtensorMap tmX, tmW, tmY;
     {
         const uint64_t dims[2] = {static_cast<uint64_t>(in), static_cast<uint64_t>(T)};
@@ -211,8 +223,6 @@ int launch_linear_tile_packed(const int* row_ptr, const uint32_t* pk_mask, const
     if (nnz_tiles > 0 && tile_packed_mode() == 1)
         return launch_linear_tile_persist(row_ptr, pk_mask, pk_off, pk_tiles, nnz_tiles, bias, X, Y, T, in,
                                           out, act, stream);
-    if (nnz_tiles > 0 && tile_packed_mode() == 2 && in % 16 == 0 && out % 16 == 0)
-        return launch_linear_expand_packed(pk_mask, pk_off, pk_tiles, bias, X, Y, T, in, out, act, stream);
     return launch_tile_common(true, row_ptr, nullptr, pk_mask, pk_off, pk_tiles, nnz_tiles, bias, X, Y,
                               T, in, out, act, stream);
 }
