@@ -91,6 +91,16 @@ NarrowPlan pick_narrow_ln(int T, int hidden, int K) {
     return p;
 }
 
+// Whether the narrow tiles take these operands: they and the LayerNorm behind them move everything in
+// 16-byte pieces.  Others keep the forms below, which read bias, gamma and beta one element at a time or
+// answer with a status.
+bool narrow_takes(const __half* X, int K, const __half* W, const __half* bias, const __half* resid,
+                  const __half* gamma, const __half* beta, const __half* out) {
+    for (const __half* p : {X, W, resid, gamma, beta, out})
+        if (!p || !aligned16(p)) return false;
+    return K % 8 == 0 && (!bias || aligned16(bias));
+}
+
 // out = LN(X W^T + bias + resid) for dense W through the narrow tiles.
 int narrow_linear_ln(const NarrowPlan& p, const __half* X, int K, const __half* W, const __half* bias,
                      const __half* resid, const __half* gamma, const __half* beta, __half* out, float* part,
@@ -234,12 +244,14 @@ int ffn_block(const et_encoder_layer_t* layer, const LayerBuffers& b, int T, __h
     } else if ((st = run_linear(layer->ffn1, b.y, b.f, T, layer->act, b, s)) != ET_OK) {
         return st;
     }
-    const NarrowPlan narrow = ffn2_dense ? pick_narrow_ln(T, layer->hidden, k2) : NarrowPlan{0, 0};
+    const __half* bias2 = reinterpret_cast<const __half*>(layer->ffn2.bias);
+    const __half* g2 = reinterpret_cast<const __half*>(layer->ln2_gamma);
+    const __half* e2 = reinterpret_cast<const __half*>(layer->ln2_beta);
+    const NarrowPlan narrow = ffn2_dense && narrow_takes(b.f, k2, w2, bias2, b.y, g2, e2, out_h)
+                                  ? pick_narrow_ln(T, layer->hidden, k2)
+                                  : NarrowPlan{0, 0};
     if (narrow.splits > 0)
-        return narrow_linear_ln(narrow, b.f, k2, w2, reinterpret_cast<const __half*>(layer->ffn2.bias), b.y,
-                                reinterpret_cast<const __half*>(layer->ln2_gamma),
-                                reinterpret_cast<const __half*>(layer->ln2_beta), out_h, b.part, T,
-                                layer->hidden, s);
+        return narrow_linear_ln(narrow, b.f, k2, w2, bias2, b.y, g2, e2, out_h, b.part, T, layer->hidden, s);
     if (ffn2_dense && ln_fused(2, T, layer->hidden, k2) && gemm_ln_applies(T, layer->hidden, k2) &&
         reinterpret_cast<const __half*>(out) != b.y) {
         // FFN2, residual and LayerNorm in one kernel
@@ -325,6 +337,7 @@ int et_encoder_layer_fwd(const et_encoder_layer_t* layer, const et_half* x, et_h
     if (!x || !out || batch <= 0 || seq <= 0) return ET_ERR_INVALID_ARG;
     if (!workspace) return ET_ERR_WORKSPACE;
     if (reinterpret_cast<uintptr_t>(workspace) & 255u) return ET_ERR_ALIGNMENT;
+    if (!et::aligned16(x) || !et::aligned16(out)) return ET_ERR_ALIGNMENT;  // before anything is launched
     const et::LayerBuffers b = et::carve(layer, batch, seq, workspace);
     if (workspace_bytes < b.total) return ET_ERR_WORKSPACE;
 
@@ -358,15 +371,16 @@ int et_encoder_layer_fwd(const et_encoder_layer_t* layer, const et_half* x, et_h
             ET_OK)
             return st;
     }
-    const et::NarrowPlan narrow = layer->o.format == ET_FMT_DENSE
+    const __half* wo = reinterpret_cast<const __half*>(layer->o.weight);
+    const __half* bo = reinterpret_cast<const __half*>(layer->o.bias);
+    const __half* g1 = reinterpret_cast<const __half*>(layer->ln1_gamma);
+    const __half* e1 = reinterpret_cast<const __half*>(layer->ln1_beta);
+    const et::NarrowPlan narrow = layer->o.format == ET_FMT_DENSE &&
+                                          et::narrow_takes(b.z, layer->vdim, wo, bo, xin, g1, e1, b.y)
                                       ? et::pick_narrow_ln(T, layer->hidden, layer->vdim)
                                       : et::NarrowPlan{0, 0};
     if (narrow.splits > 0) {
-        if ((st = et::narrow_linear_ln(narrow, b.z, layer->vdim,
-                                       reinterpret_cast<const __half*>(layer->o.weight),
-                                       reinterpret_cast<const __half*>(layer->o.bias), xin,
-                                       reinterpret_cast<const __half*>(layer->ln1_gamma),
-                                       reinterpret_cast<const __half*>(layer->ln1_beta), b.y, b.part, T,
+        if ((st = et::narrow_linear_ln(narrow, b.z, layer->vdim, wo, bo, xin, g1, e1, b.y, b.part, T,
                                        layer->hidden, s)) != ET_OK)
             return st;
     } else if (layer->o.format == ET_FMT_DENSE && et::ln_fused(1, T, layer->hidden, layer->vdim) &&
@@ -439,6 +453,7 @@ int et_encoder_after_attention_fwd(const et_encoder_layer_t* layer, const void* 
     if (!x || !out || !attn_sum || batch <= 0 || seq <= 0) return ET_ERR_INVALID_ARG;
     if (!workspace) return ET_ERR_WORKSPACE;
     if (reinterpret_cast<uintptr_t>(workspace) & 255u) return ET_ERR_ALIGNMENT;
+    if (!et::aligned16(x) || !et::aligned16(out) || !et::aligned16(attn_sum)) return ET_ERR_ALIGNMENT;
     const et::LayerBuffers b = et::carve(layer, batch, seq, workspace);
     if (workspace_bytes < b.total) return ET_ERR_WORKSPACE;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
@@ -467,7 +482,7 @@ int et_encoder_ffn_fwd(const et_encoder_layer_t* layer, const et_half* y, et_hal
     if (!y || !out || batch <= 0 || seq <= 0) return ET_ERR_INVALID_ARG;
     if (!workspace) return ET_ERR_WORKSPACE;
     if (reinterpret_cast<uintptr_t>(workspace) & 255u) return ET_ERR_ALIGNMENT;
-    if (!et::aligned16(y)) return ET_ERR_ALIGNMENT;
+    if (!et::aligned16(y) || !et::aligned16(out)) return ET_ERR_ALIGNMENT;
     et::LayerBuffers b = et::carve(layer, batch, seq, workspace);
     if (workspace_bytes < b.total) return ET_ERR_WORKSPACE;
     b.y = const_cast<__half*>(reinterpret_cast<const __half*>(y));  // read only

@@ -290,6 +290,9 @@ int launch_skip_layernorm_partials(const float* partials, int nsplit, size_t spl
     if (!partials || !gamma || !beta || !out || rows <= 0 || size <= 0 || nsplit <= 0)
         return ET_ERR_INVALID_ARG;
     if (size % 8 || size > LNP_MAX_WARPS * 32 * 8 || nsplit > 4) return ET_ERR_SHAPE;
+    if (!aligned16(partials) || !aligned16(gamma) || !aligned16(beta) || !aligned16(out) ||
+        (bias && !aligned16(bias)) || (skip && !aligned16(skip)))
+        return ET_ERR_ALIGNMENT;
     const int threads = (size / 8 + 31) / 32 * 32;
     auto go = [&](auto kern) {
         return launch_kernel(kern, dim3(rows), dim3(threads), 0, stream, partials, split_stride, bias, skip,

@@ -136,3 +136,51 @@ def test_attention_fuse_o_single_launch_argument_checks(et):
     assert call(emdim=770) == -3
     assert call(Q=0x1008) == -2
 
+
+
+def _layer_desc(et, **pointers):
+    """A dense 768-wide layer whose pointers are made up: for calls that must be refused on the host."""
+    d = et.EncoderLayerDesc()
+    for i, (lin, inn, out) in enumerate(((d.qkv, 768, 2304), (d.o, 768, 768), (d.ffn1, 768, 3072),
+                                         (d.ffn2, 3072, 768))):
+        lin.in_, lin.out, lin.weight, lin.bias = inn, out, 0x100000 * (i + 1), 0x1000 * (i + 1)
+    for i, name in enumerate(("ln1_gamma", "ln1_beta", "ln2_gamma", "ln2_beta")):
+        setattr(d, name, 0x10000 * (i + 1))
+    d.hidden, d.nhead, d.kdim, d.vdim, d.ff, d.act = 768, 12, 768, 768, 3072, 2
+    for k, v in pointers.items():
+        setattr(d, k, v)
+    return d
+
+
+def test_misaligned_layer_tensors_are_refused_before_a_launch(et):
+    """The layer's kernels move x, its output and the all-reduced sum in 16-byte pieces: each is checked on
+    the host at the entry, before the first kernel."""
+    lib = et.lib()
+    d = _layer_desc(et)
+    P, Z = ctypes.c_void_p, ctypes.c_size_t
+    ref, ws, big = ctypes.byref(d), P(0x40000000), Z(1 << 40)
+    before = lib.et_launch_count()
+    for x, out in ((0x2000008, 0x3000000), (0x2000000, 0x3000008), (0x2000000, 0x3000002)):
+        assert lib.et_encoder_layer_fwd(ref, P(x), P(out), 1, 128, 0, None, None, ws, big, None) == -2
+        assert lib.et_encoder_ffn_fwd(ref, P(x), P(out), 1, 128, ws, big, None) == -2
+        for f32 in (0, 1):
+            assert lib.et_encoder_after_attention_fwd(ref, P(0x5000000), f32, P(x), P(out), 1, 128, ws, big,
+                                                      None) == -2
+    for f32 in (0, 1):
+        assert lib.et_encoder_after_attention_fwd(ref, P(0x5000008), f32, P(0x2000000), P(0x3000000), 1, 128,
+                                                  ws, big, None) == -2
+    assert lib.et_launch_count() == before
+
+
+def test_partial_sum_layernorm_refuses_misaligned_vectors(et):
+    """bias, gamma and beta of a LayerNorm that adds up fp32 sums are read 16 bytes at a time."""
+    lib = et.lib()
+    P, Z = ctypes.c_void_p, ctypes.c_size_t
+    for name in ("ln1_gamma", "ln1_beta"):
+        d = _layer_desc(et, **{name: 0x10002})
+        assert lib.et_encoder_after_attention_fwd(ctypes.byref(d), P(0x5000000), 1, P(0x2000000), P(0x3000000), 1,
+                                                  128, P(0x40000000), Z(1 << 40), None) == -2
+    d = _layer_desc(et)
+    d.o.bias = 0x1004
+    assert lib.et_encoder_after_attention_fwd(ctypes.byref(d), P(0x5000000), 1, P(0x2000000), P(0x3000000), 1, 128,
+                                              P(0x40000000), Z(1 << 40), None) == -2

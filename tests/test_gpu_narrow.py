@@ -59,3 +59,39 @@ def test_layer_with_few_row_blocks(et, orc, cuda, batch, seq, hidden, nhead, ff)
     ref = orc.encoder_layer(x.astype(np.float32), w, batch, seq, nhead, 2, 2, None, vl)
     assert_close(y.float().cpu().numpy(), ref, f"layer {batch}x{seq}x{hidden}")
     assert torch.equal(y, stack.forward(_dev(x, cuda), et.MASK_PADDING, None, _dev(vl, cuda)))
+
+
+@pytest.mark.parametrize("batch,seq", [(1, 128), (5, 77)])
+def test_layer_with_vectors_off_16_byte_boundaries(et, orc, cuda, batch, seq):
+    """bias, gamma and beta of the O projection and FFN2 may lie anywhere: the fused kernel reads them one
+    element at a time, and a layer with few row blocks must not lose that to the narrow tiles."""
+    import torch
+    hidden, nhead, ff = 768, 12, 3072
+    w = et.synth.encoder_layer_weights(83, 0, hidden, ff, bias_std=0.02, ln_noise=0.05, fast=True)
+    x = et.synth.normal_fast(83, 9, (batch * seq, hidden), 1.0)
+    layer = et.EncoderLayer(w, nhead, et.ACT_GELU, device=cuda)
+    keep = []
+
+    def shifted(a, by):
+        t = torch.zeros(a.size + 8, dtype=torch.float16, device=cuda)
+        t[by:by + a.size] = torch.from_numpy(np.ascontiguousarray(a, np.float16)).to(cuda)
+        keep.append(t)
+        return t.data_ptr() + 2 * by
+
+    for i, n in enumerate(("ln1_gamma", "ln1_beta", "ln2_gamma", "ln2_beta")):
+        setattr(layer.desc, n, shifted(w[n.replace("amma", "").replace("eta", "")], i + 1))
+    layer.desc.o.bias = shifted(w["bo"], 5)
+    layer.desc.ffn2.bias = shifted(w["b2"], 6)
+    stack = et.EncoderStack([layer], batch, seq, device=cuda)
+    y = stack.forward(_dev(x, cuda)).clone()
+    assert et.device_error() == 0
+    ref = orc.encoder_layer(x.astype(np.float32), w, batch, seq, nhead, 2, 0, None, None)
+    assert_close(y.float().cpu().numpy(), ref, f"shifted vectors {batch}x{seq}")
+    # an output off a boundary is refused, and nothing is launched
+    before = et.lib().et_launch_count()
+    out = torch.zeros(batch * seq * hidden + 8, dtype=torch.float16, device=cuda)[4:4 + batch * seq * hidden]
+    ws = torch.empty(et.lib().et_encoder_layer_workspace_bytes(ctypes.byref(layer.desc), batch, seq),
+                     dtype=torch.uint8, device=cuda)
+    with pytest.raises(et.EtError, match="-2"):
+        layer.forward(_dev(x, cuda), out, batch, seq, ws)
+    assert et.lib().et_launch_count() == before and et.device_error() == 0
