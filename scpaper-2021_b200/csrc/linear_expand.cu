@@ -173,6 +173,46 @@ struct PackedExpander {
     }
 };
 
+// Output feature n of one token from the stored entries alone.  The expanded operand multiplies every
+// activation, by zero where nothing is stored, which is the same sum as long as the token is finite; the
+// epilogue asks here for elements that are not, so that an infinity or NaN reaches exactly the outputs
+// that store a weight for it (a vector or a tile is stored whole).
+template <int FMT>
+__device__ __noinline__ float stored_product(const int* idx0, const int* idx1, const __half* data, int in,
+                                             int n, const __half* x) {
+    float acc = 0.f;
+    auto dot16 = [&](const __half* w, int k) {
+        for (int j = 0; j < 16; ++j) acc += __half2float(__ldg(w + j)) * __half2float(__ldcg(x + k + j));
+    };
+    if (FMT == FMT_CSRM) {
+        for (int e = __ldg(idx0 + n); e < __ldg(idx0 + n + 1); ++e) {
+            const int k = __ldg(idx1 + e);
+            if (k >= 0 && k < in) acc += __half2float(__ldg(data + e)) * __half2float(__ldcg(x + k));
+        }
+    } else if (FMT == FMT_VEC) {
+        const int npart = in >> 4;
+        const int* tidx = idx0 + static_cast<size_t>(n >> 4) * (npart + 1);
+        for (int p = 0; p < npart; ++p)
+            for (int i = __ldg(tidx + p); i < __ldg(tidx + p + 1); ++i)
+                if ((__ldg(idx1 + i) & 15) == (n & 15)) dot16(data + static_cast<size_t>(i) * 16, p * 16);
+    } else {
+        const int nchunk = (in + 63) >> 6, r4 = ((n >> 4) & 7) * 4, row = n & 15;
+        for (int kb = 0; kb < nchunk; ++kb) {
+            const size_t at = static_cast<size_t>(n >> 7) * nchunk + kb;
+            const uint32_t m = __ldg(reinterpret_cast<const uint32_t*>(idx0) + at);
+            int slot = __ldg(idx1 + at) + __popc(m & ((1u << r4) - 1u));
+            for (int c = 0; c < 4; ++c) {
+                if (!((m >> (r4 + c)) & 1u)) continue;
+                const __half* w = data + static_cast<size_t>(slot++) * 256 + row * 16;
+                for (int j = 0; j < 16; ++j)  // (halves swapped in rows 4-7 and 12-15)
+                    acc += __half2float(__ldg(w + (j ^ (((row >> 2) & 1) * 8)))) *
+                           __half2float(__ldcg(x + kb * 64 + c * 16 + j));
+            }
+        }
+    }
+    return acc;
+}
+
 template <int FMT, int BN>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 linear_expand_kernel(const __grid_constant__ CUtensorMap tmX, const ExpandArgs g) {
@@ -423,6 +463,7 @@ linear_expand_kernel(const __grid_constant__ CUtensorMap tmX, const ExpandArgs g
             constexpr int NG = BN / GROUP;
             uint8_t* tile = sA + w * 4096;
             const bool any_dup = FMT == FMT_CSRM && *reinterpret_cast<volatile int*>(s_any_dup) != 0;
+            bool odd = false;  // a row of this thread is not finite: see below
             for (int u = half; u < mb * NG; u += 2) {
                 const int tb = u / NG, cg = u - tb * NG;
                 const int n_base = n0 + cg * GROUP;
@@ -434,22 +475,7 @@ linear_expand_kernel(const __grid_constant__ CUtensorMap tmX, const ExpandArgs g
                     uint32_t r[32];
                     tmem_ld32(addr + h * 32, r);
                     tmem_ld_wait_regs(r);
-                    if (FMT == FMT_CSRM && any_dup) {
-                        const int m = row0 + lane;
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) {
-                            const int nl = cg * GROUP + h * 32 + j;
-                            if (!reinterpret_cast<volatile int*>(s_dup)[nl]) continue;
-                            float acc = 0.f;
-                            for (int e = s_ptr[nl]; m < g.T && e < s_ptr[nl + 1]; ++e) {
-                                const int k = __ldg(g.idx1 + e);
-                                if (k >= 0 && k < g.in)
-                                    acc += __half2float(__ldg(g.data + e)) *
-                                           __half2float(__ldcg(g.X + static_cast<size_t>(m) * g.in + k));
-                            }
-                            r[j] = __float_as_uint(acc);
-                        }
-                    }
+                    odd = odd || (r[0] & 0x7f800000u) == 0x7f800000u;
                     const float* b32 = s_bias + cg * GROUP + h * 32;
                     if (g.act == ET_ACT_GELU) stage_f16_chunk<ET_ACT_GELU>(r, b32, tile + lane * 128, h, lane);
                     else if (g.act == ET_ACT_RELU) stage_f16_chunk<ET_ACT_RELU>(r, b32, tile + lane * 128, h, lane);
@@ -475,6 +501,37 @@ linear_expand_kernel(const __grid_constant__ CUtensorMap tmX, const ExpandArgs g
                 }
                 __syncwarp();
             }
+            // Elements to be summed again from the stored entries: rows of the weight that hold a column
+            // twice, and whatever is not finite.  (An activation that is not finite leaves no element of its
+            // row finite, so one of 32 tells.  A pass of its own: inside the loop above it cost 3 % of
+            // 1024 -> 3072 at 3072 tokens.)
+            if (any_dup || __any_sync(0xffffffffu, odd))
+                for (int u = half; u < mb * NG; u += 2) {
+                    const int tb = u / NG, cg = u - tb * NG;
+                    const int row0 = m0 + tb * BM + q * 32, m = row0 + lane;
+                    if (row0 >= g.T || n0 + cg * GROUP >= g.out) continue;
+                    for (int h = 0; h < GROUP / 32; ++h) {
+                        const int nl = cg * GROUP + h * 32;  // first of 32 columns
+                        uint32_t r[32];
+                        __syncwarp();
+                        tmem_ld32(tmem_base + tb * BN + nl + (static_cast<uint32_t>(q * 32) << 16), r);
+                        tmem_ld_wait_regs(r);
+                        uint32_t redo = 0;
+                        if (any_dup)
+                            redo = __ballot_sync(0xffffffffu, reinterpret_cast<volatile int*>(s_dup)[nl + lane]);
+#pragma unroll
+                        for (int j = 0; j < 32; ++j)
+                            redo |= (r[j] & 0x7f800000u) == 0x7f800000u ? 1u << j : 0u;
+                        for (; m < g.T && redo != 0; redo &= redo - 1) {
+                            const int j = __ffs(redo) - 1, n = n0 + nl + j;
+                            if (n >= g.out) break;
+                            const float y = stored_product<FMT>(g.idx0, g.idx1, g.data, g.in, n,
+                                                                g.X + static_cast<size_t>(m) * g.in) +
+                                            s_bias[nl + j];
+                            g.Y[static_cast<size_t>(m) * g.out + n] = __float2half_rn(apply_act(y, g.act));
+                        }
+                    }
+                }
         }
     }
 

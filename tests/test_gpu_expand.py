@@ -100,3 +100,57 @@ def test_packed_tiles(et, orc, cuda, T, inn, out, sparsity):
     _check(ys[0], orc.linear_dense(x, w, b, 2), f"packed {T}x{inn}x{out} s={sparsity}")
     # the products of absent tiles add exact zeros: the same bits
     assert torch.equal(ys[0], ys[1])
+
+
+def _with_infinities(et, seed, T, inn):
+    """Activations with infinities of both signs and NaN in a few (token, feature) places."""
+    x = et.synth.normal_fast(seed, 1, (T, inn), 1.0)
+    for i, t in enumerate(range(0, T, 3)):
+        x[t, (37 * i + 5) % inn] = (np.inf, -np.inf, np.nan, 65504.0)[i % 4]
+        if i % 5 == 0:
+            x[t, (11 * i) % inn] = np.inf
+    return x
+
+
+def _same_with_infinities(y, ref, what):
+    y, ref = y.float().cpu().numpy(), ref.astype(np.float32)
+    assert np.array_equal(np.isnan(y), np.isnan(ref)), f"{what}: NaN in other places"
+    inf = np.isinf(ref)
+    assert np.array_equal(np.isinf(y), inf) and np.array_equal(y[inf], ref[inf]), f"{what}: infinities"
+    fin = np.isfinite(ref)
+    # the fp16 rounding of the output and, per token, fp32 sums of terms as large as 65504 * |w|
+    scale = np.abs(np.where(fin, ref, 0)).max(axis=1, keepdims=True)
+    d = np.abs(np.where(fin, y, 0) - np.where(fin, ref, 0))
+    assert (d <= 2.0 ** -10 * scale + 6e-4).all(), f"{what}: {d.max()}"
+
+
+@pytest.mark.parametrize("T,inn,out", [(40, 256, 48), (200, 2048, 112), (1100, 768, 272)])
+def test_an_infinity_reaches_only_outputs_that_store_a_weight_for_it(et, orc, cuda, T, inn, out):
+    """Expanded operands hold zeros where nothing is stored, and 0 * inf is NaN: the product must still be the
+    sum over stored entries, whichever kernel the token count selects for packed tiles."""
+    import ctypes
+    x = _with_infinities(et, 75, T, inn)
+    xf, b = x.astype(np.float32), et.synth.normal_fast(75, 3, (out,), 0.1)
+    w = et.synth.normal_fast(75, 2, (out, inn), 0.05)
+    d = lambda a: _dev(a, cuda)
+    with np.errstate(invalid="ignore"):
+        wv = et.synth.prune_1x16(w, 75, 6, 0.8)
+        ti, ri, dv = et.synth.dense_to_1x16(wv)
+        y = et.linear_1x16(d(x), d(ti), d(ri), d(dv), out, d(b), 0)
+        _same_with_infinities(y, orc.linear_1x16(xf, ti, ri, dv, out, b, 0), "1x16")
+        wc = w * (et.synth.uniform(75, 7, out * inn).reshape(out, inn) >= 0.9)
+        ip, ix, dc = et.synth.dense_to_csr(wc)
+        y = et.linear_csr(d(x), d(ip), d(ix), d(dc), out, d(b), 0)
+        _same_with_infinities(y, orc.linear_csr(xf, ip, ix, dc, out, b, 0), "csr")
+        wt = et.synth.prune_tiles(w, 75, 4, 0.8)
+        rp, ro, tiles = et.synth.dense_to_tile(wt)
+        ref = orc.linear_tile(xf, rp, ro, tiles, out, b, 0)
+        pk = et.PackedTiles(rp, ro, tiles, inn, out, cuda)
+        for mode in (-1, 2, 0):  # automatic, expanded tiles, one product per stored tile
+            et.lib().et_debug_set_tile_persist(ctypes.c_int(mode))
+            try:
+                y = et.linear_tile_packed(d(x), pk, d(b), 0)
+            finally:
+                et.lib().et_debug_set_tile_persist(ctypes.c_int(-1))
+            _same_with_infinities(y, ref, f"packed tiles, mode {mode}")
+    assert et.device_error() == 0
