@@ -258,13 +258,13 @@ __device__ __forceinline__ void attention_cta(const CUtensorMap& tmQ, const CUte
             const uint32_t v_lo =
                 ((smem_u32(sV) & 0x3FFFFu) >> 4) | (static_cast<uint32_t>(ATOM_BYTES >> 4) << 16);
             const int ksteps = a.dh_qk >> 4;
-            bool ok = mbar_wait_bounded(q_full, 0, abort_flag);
+            bool ok = mbar_wait_bounded_warp(q_full, 0, abort_flag);
             // S_j = Q.K_j^T; the score block is free as soon as the softmax warps hold it in
             // registers, so S_{j+1} is issued BEFORE P_j.V_j and runs under softmax(j).
             auto issue_s = [&](int j) -> bool {
                 const uint32_t ph = j & 1;
-                if (!(mbar_wait_bounded(k_full, ph, abort_flag) &&
-                      mbar_wait_bounded(s_free, ph ^ 1, abort_flag)))
+                if (!(mbar_wait_bounded_warp(k_full, ph, abort_flag) &&
+                      mbar_wait_bounded_warp(s_free, ph ^ 1, abort_flag)))
                     return false;
                 tc_fence_after_sync();
                 if (leader) {
@@ -285,8 +285,8 @@ __device__ __forceinline__ void attention_cta(const CUtensorMap& tmQ, const CUte
             for (int j = 0; ok && j < n_kv; ++j) {
                 const uint32_t ph = j & 1;
                 if (j + 1 < n_kv) ok = issue_s(j + 1);
-                ok = ok && mbar_wait_bounded(p_full, ph, abort_flag) &&
-                     mbar_wait_bounded(v_full, ph, abort_flag);
+                ok = ok && mbar_wait_bounded_warp(p_full, ph, abort_flag) &&
+                     mbar_wait_bounded_warp(v_full, ph, abort_flag);
                 if (!ok) break;
                 tc_fence_after_sync();
                 if (leader) {
@@ -303,8 +303,8 @@ __device__ __forceinline__ void attention_cta(const CUtensorMap& tmQ, const CUte
             if (FUSED && ok) {
                 // the barriers are invalidated after this piece of work: every arrival a commit
                 // has scheduled must have happened by then
-                ok = mbar_wait_bounded(k_empty, (n_kv - 1) & 1, abort_flag) &&
-                     mbar_wait_bounded(v_empty, (n_kv - 1) & 1, abort_flag);
+                ok = mbar_wait_bounded_warp(k_empty, (n_kv - 1) & 1, abort_flag) &&
+                     mbar_wait_bounded_warp(v_empty, (n_kv - 1) & 1, abort_flag);
             }
             if (!ok && leader) report_error(a.err_word, abort_flag, DEV_TIMEOUT_ATTN_MMA);
             __syncwarp();

@@ -246,9 +246,9 @@ attention_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         bool ok = true;
         auto issue_s = [&]() -> bool {
             const int s = gs & 1;
-            if ((js == 0 && !mbar_wait_bounded(q_full, item_s & 1, abort_flag)) ||
-                !mbar_wait_bounded(&k_full[s], (gs >> 1) & 1, abort_flag) ||
-                !mbar_wait_bounded(s_free, (gs & 1) ^ 1, abort_flag))
+            if ((js == 0 && !mbar_wait_bounded_warp(q_full, item_s & 1, abort_flag)) ||
+                !mbar_wait_bounded_warp(&k_full[s], (gs >> 1) & 1, abort_flag) ||
+                !mbar_wait_bounded_warp(s_free, (gs & 1) ^ 1, abort_flag))
                 return false;
             tc_fence_after_sync();
             const bool last = js + 1 == ws.n_kv;
@@ -277,8 +277,8 @@ attention_rows_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             for (int j = 0; ok && j < wo.n_kv; ++j, ++go) {
                 const int s = go & 1;
                 if (more_s) ok = issue_s();  // runs under this block's softmax
-                ok = ok && mbar_wait_bounded(&v_full[s], (go >> 1) & 1, abort_flag) &&
-                     mbar_wait_bounded(p_full, go & 1, abort_flag);
+                ok = ok && mbar_wait_bounded_warp(&v_full[s], (go >> 1) & 1, abort_flag) &&
+                     mbar_wait_bounded_warp(p_full, go & 1, abort_flag);
                 if (!ok) break;
                 tc_fence_after_sync();
                 if (leader) {

@@ -234,8 +234,8 @@ attention_vo_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             const int ksteps = a.dh_qk >> 4;
             auto issue_s = [&](int t) -> bool {
                 const int s = t & (qk_stages - 1);
-                if (!mbar_wait_bounded(&qk_full[s], (qk_stages == 2 ? t >> 1 : t) & 1, abort_flag) ||
-                    !mbar_wait_bounded(&s_free[t & 1], ((t >> 1) & 1) ^ 1, abort_flag))
+                if (!mbar_wait_bounded_warp(&qk_full[s], (qk_stages == 2 ? t >> 1 : t) & 1, abort_flag) ||
+                    !mbar_wait_bounded_warp(&s_free[t & 1], ((t >> 1) & 1) ^ 1, abort_flag))
                     return false;
                 tc_fence_after_sync();
                 const uint32_t q_lo = qk_lo + s * (qk_stage_bytes >> 4);
@@ -259,9 +259,9 @@ attention_vo_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                 if (t + 1 < n_task) ok = issue_s(t + 1);
                 if (!ok) break;
                 if (in_head >= per_head - n_kv) {
-                    ok = mbar_wait_bounded(p_full, t_b & 1, abort_flag);
+                    ok = mbar_wait_bounded_warp(p_full, t_b & 1, abort_flag);
                     for (int half = 0; ok && half < 2; ++half) {
-                        ok = mbar_wait_bounded(&vo_full[v], vph, abort_flag);
+                        ok = mbar_wait_bounded_warp(&vo_full[v], vph, abort_flag);
                         if (!ok) break;
                         tc_fence_after_sync();
                         if (leader) {

@@ -183,6 +183,18 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
     return false;
 }
 
+// The same by a whole warp that goes on as one (the warps that issue tensor-core products).  The lanes vote on
+// every poll: lanes that see the barrier complete and lanes that see *abort_flag first would part otherwise,
+// and wait for each other at a warp barrier for good.
+__device__ __forceinline__ bool mbar_wait_bounded_warp(uint64_t* bar, uint32_t parity,
+                                                       volatile int* abort_flag) {
+    for (uint32_t it = 0; it < ET_SPIN_LIMIT; ++it) {
+        if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+        if ((it & 255u) == 255u && __any_sync(0xffffffffu, *abort_flag)) return false;
+    }
+    return false;
+}
+
 // Same contract for waits that are expected to last long (an epilogue waiting for a whole
 // main loop): the warp sleeps between polls so that it does not compete for issue slots
 // with the producer and MMA-issuing threads that share its scheduler.

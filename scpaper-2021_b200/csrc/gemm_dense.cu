@@ -234,14 +234,14 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             // (an empty K slice issues no MMA: the commit below then arrives at once and the
             // epilogue writes zeros)
             // the epilogue must have drained this accumulator's previous tile
-            if (!mbar_wait_bounded(&acc_empty[buf], use_ph ^ 1, abort_flag)) {
+            if (!mbar_wait_bounded_warp(&acc_empty[buf], use_ph ^ 1, abort_flag)) {
                 ok = false;
                 break;
             }
             tc_fence_after_sync();
             const uint32_t d_tmem = tmem_base + buf * BN;
             for (int i = 0; i < c.num_kb; ++i) {
-                if (!mbar_wait_bounded(&full_bar[s], ph, abort_flag)) {
+                if (!mbar_wait_bounded_warp(&full_bar[s], ph, abort_flag)) {
                     ok = false;
                     break;
                 }

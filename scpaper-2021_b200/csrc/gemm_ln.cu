@@ -158,7 +158,7 @@ gemm_ln_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         int s = 0;
         uint32_t ph = 0;
         for (int i = 0; i < num_kb; ++i) {
-            if (!mbar_wait_bounded(&full_bar[s], ph, abort_flag)) {
+            if (!mbar_wait_bounded_warp(&full_bar[s], ph, abort_flag)) {
                 mma_ok = false;
                 break;
             }

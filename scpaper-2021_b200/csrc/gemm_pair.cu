@@ -219,14 +219,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 const int buf = PERSIST ? (tile_iter & 1) : 0;
                 const uint32_t use_ph = (tile_iter >> 1) & 1;
                 // both CTAs' epilogues must have drained this accumulator's previous tile
-                if (PERSIST && !mbar_wait_bounded(&acc_empty[buf], use_ph ^ 1, abort_flag)) {
+                if (PERSIST && !mbar_wait_bounded_warp(&acc_empty[buf], use_ph ^ 1, abort_flag)) {
                     ok = false;
                     break;
                 }
                 tc_fence_after_sync();
                 const uint32_t d_tmem = tmem_base + buf * BN;
                 for (int i = 0; i < num_kb; ++i) {
-                    if (!mbar_wait_bounded(&full_bar[s], ph, abort_flag)) {
+                    if (!mbar_wait_bounded_warp(&full_bar[s], ph, abort_flag)) {
                         ok = false;
                         break;
                     }

@@ -213,14 +213,14 @@ gemm_pair_ln_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             for (int t = cluster; ok && t < tiles; t += nclusters, ++it) {
                 const int buf = it & 1;
                 // both CTAs' epilogues must have drained this accumulator's previous tile
-                if (!mbar_wait_bounded(&acc_empty[buf], ((it >> 1) & 1) ^ 1, abort_flag)) {
+                if (!mbar_wait_bounded_warp(&acc_empty[buf], ((it >> 1) & 1) ^ 1, abort_flag)) {
                     ok = false;
                     break;
                 }
                 tc_fence_after_sync();
                 const uint32_t d_tmem = tmem_base + buf * PL_BN;
                 for (int i = 0; i < num_kb; ++i) {
-                    if (!mbar_wait_bounded(&full_bar[s], ph, abort_flag)) {
+                    if (!mbar_wait_bounded_warp(&full_bar[s], ph, abort_flag)) {
                         ok = false;
                         break;
                     }

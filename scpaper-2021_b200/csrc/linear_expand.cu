@@ -312,7 +312,7 @@ linear_expand_kernel(const __grid_constant__ CUtensorMap tmX, const ExpandArgs g
         uint32_t ph = 0, bph = 0;
         bool ok = true;
         for (int c = 0; ok && c < nchunk; ++c) {
-            if (!mbar_wait_bounded(&b_full[buf], bph, abort_flag)) {
+            if (!mbar_wait_bounded_warp(&b_full[buf], bph, abort_flag)) {
                 ok = false;
                 break;
             }
@@ -320,7 +320,7 @@ linear_expand_kernel(const __grid_constant__ CUtensorMap tmX, const ExpandArgs g
             uint32_t b_lo = b_base + ((buf * buf_bytes) >> 4);
             for (int kb = c * g.ckb; ok && kb < kb_end; ++kb, b_lo += (BN * 128) >> 4) {
                 for (int tb = 0; tb < mb; ++tb) {
-                    if (!mbar_wait_bounded(&a_full[s], ph, abort_flag)) {
+                    if (!mbar_wait_bounded_warp(&a_full[s], ph, abort_flag)) {
                         ok = false;
                         break;
                     }

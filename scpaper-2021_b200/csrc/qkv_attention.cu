@@ -190,7 +190,7 @@ qkv_attention_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
         uint32_t ph = 0;
         bool ok = true;
         for (int i = 0; i < nkb; ++i) {
-            if (!mbar_wait_bounded(&full_bar[s], ph, abort_flag)) {
+            if (!mbar_wait_bounded_warp(&full_bar[s], ph, abort_flag)) {
                 ok = false;
                 break;
             }
@@ -216,7 +216,7 @@ qkv_attention_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
                 QA_TL(5);
             }
             __syncwarp();
-            ok = mbar_wait_bounded(qkv_ready, 0, abort_flag);
+            ok = mbar_wait_bounded_warp(qkv_ready, 0, abort_flag);
         }
         if (ok) {
             tc_fence_after_sync();
@@ -230,7 +230,7 @@ qkv_attention_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
                 mma_commit(s_full);
             }
             __syncwarp();
-            ok = mbar_wait_bounded(p_full, 0, abort_flag);
+            ok = mbar_wait_bounded_warp(p_full, 0, abort_flag);
             if (ok) {
                 tc_fence_after_sync();
                 if (leader) {
