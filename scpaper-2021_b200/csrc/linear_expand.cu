@@ -31,6 +31,8 @@ enum : int { FMT_VEC = 0, FMT_PACKED = 1, FMT_CSRM = 2 };
 constexpr int X_MAX_A = 8;                       // activation stages at most
 constexpr int X_MAX_B = 4;                       // weight buffers at most
 constexpr int X_MAX_MB = 8;                      // token blocks per CTA at most
+constexpr int X_CSR_A = 4;                       // CSR: activation stages,
+constexpr int X_CSR_BYTES = 128 * 1024;          // and bytes of expanded columns at most
 constexpr int X_EXP_WARPS = EPI_WARPS;           // expander / epilogue warps
 constexpr int X_EXP_THREADS = 32 * X_EXP_WARPS;
 constexpr int X_ROW_LIST = 128 + 1;
@@ -544,16 +546,21 @@ linear_expand_kernel(const __grid_constant__ CUtensorMap tmX, const ExpandArgs g
 template <int FMT, int BN>
 int launch_bn(const CUtensorMap& tmX, ExpandArgs& a, cudaStream_t stream) {
     const int buf = a.ckb * BN * 128;
-    const int misc = 256 + BN * 4 + (FMT == FMT_CSRM ? (X_ROW_LIST + BN) * 4 : 0);
+    constexpr int misc = 256 + BN * 4 + (FMT == FMT_CSRM ? (X_ROW_LIST + BN) * 4 : 0);
     const int smem = a.na * A_STAGE_BYTES + a.nbuf * buf + misc + 1024;
     auto kern = linear_expand_kernel<FMT, BN>;
-    static std::atomic<int> attr_bytes[64] = {};
+    // once, to the most that any width needs: two threads that each raised it to their own size could leave
+    // the smaller one standing
+    constexpr int most = (FMT == FMT_CSRM ? X_CSR_A * A_STAGE_BYTES + X_CSR_BYTES
+                                          : X_MAX_A * A_STAGE_BYTES + X_MAX_B * 128 * 128) + misc + 1024;
+    static_assert(most <= 227 * 1024, "shared memory budget exceeded");
+    static std::atomic<bool> attr_set[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
-    if (dev >= 0 && dev < 64 && attr_bytes[dev] < smem) {
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+    if (dev >= 0 && dev < 64 && !attr_set[dev]) {
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess)
             return ET_ERR_CUDA;
-        attr_bytes[dev] = smem;
+        attr_set[dev] = true;
     }
     const long panels = (a.out + BN - 1) / BN;
     return launch_kernel(kern, dim3(static_cast<unsigned>(panels * a.groups)), dim3(GEMM_THREADS), smem,
@@ -598,10 +605,10 @@ int launch_expand(ExpandArgs a, cudaStream_t stream) {
     while (cols < a.mb * bn) cols <<= 1;
     a.tmem_cols = cols;
     if (FMT == FMT_CSRM) {
-        const int fit = (128 * 1024) / (bn * 128);  // 128 KB of expanded columns
+        const int fit = X_CSR_BYTES / (bn * 128);
         a.ckb = nkb < fit ? nkb : fit;
         a.nbuf = 1;
-        a.na = 4;
+        a.na = X_CSR_A;
     } else {
         a.ckb = 128 / bn;  // eight warps, one (row set, K block) item each
         a.nbuf = X_MAX_B;

@@ -154,3 +154,40 @@ def test_an_infinity_reaches_only_outputs_that_store_a_weight_for_it(et, orc, cu
                 et.lib().et_debug_set_tile_persist(ctypes.c_int(-1))
             _same_with_infinities(y, ref, f"packed tiles, mode {mode}")
     assert et.device_error() == 0
+
+
+def test_first_calls_of_narrow_and_wide_layers_from_many_threads(et, cuda):
+    """The kernel's shared-memory limit belongs to the process: whichever thread's first call comes last, wide
+    layers (192 KB) must still launch beside narrow ones."""
+    import subprocess
+    import sys
+    from conftest import ROOT
+    code = """
+import importlib, sys, threading
+sys.path.insert(0, %r)
+import torch
+et = importlib.import_module("scpaper-2021_b200")
+def layer(inn):
+    out = 64
+    ip = torch.arange(out + 1, dtype=torch.int32, device="cuda") * 400
+    ix = torch.arange(400, dtype=torch.int32, device="cuda").repeat(out)
+    return (torch.ones(8, inn, device="cuda").half(), ip, ix, torch.ones(400 * out, device="cuda").half(), out)
+layers = [layer(i) for i in (8192, 512, 1024, 4096) * 4]
+et.lib()
+start, bad = threading.Barrier(len(layers)), []
+def work(a):
+    start.wait()
+    try:
+        for _ in range(20):
+            et.linear_csr(*a)
+    except Exception as e:
+        bad.append(e)
+ts = [threading.Thread(target=work, args=(a,)) for a in layers]
+[t.start() for t in ts]; [t.join() for t in ts]
+y = et.linear_csr(*layers[0])
+torch.cuda.synchronize()
+assert not bad, bad
+assert (y == 400).all() and et.device_error() == 0
+""" % ROOT
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=180)
+    assert r.returncode == 0, r.stderr[-2000:]
