@@ -649,7 +649,7 @@ int et_linear_1x16_fwd(const int32_t* tile_idx, const int32_t* row_idx, const et
         return ET_ERR_INVALID_ARG;
     if (nvec > 0 && (!row_idx || !data)) return ET_ERR_INVALID_ARG;
     if (act < ET_ACT_NONE || act > ET_ACT_GELU) return ET_ERR_INVALID_ARG;
-    if (in % 16 || out % 16) return ET_ERR_SHAPE;
+    if (in % 16 || out % 16 || T > 65535 * 128) return ET_ERR_SHAPE;
     if (!et::aligned16(X) || !et::aligned16(Y) || (data && !et::aligned16(data)))
         return ET_ERR_ALIGNMENT;
     et::ExpandArgs a = {};

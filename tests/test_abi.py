@@ -184,3 +184,11 @@ def test_partial_sum_layernorm_refuses_misaligned_vectors(et):
     d.o.bias = 0x1004
     assert lib.et_encoder_after_attention_fwd(ctypes.byref(d), P(0x5000000), 1, P(0x2000000), P(0x3000000), 1, 128,
                                               P(0x40000000), Z(1 << 40), None) == -2
+
+
+def test_1x16_refuses_more_than_65535_token_blocks(et):
+    lib = et.lib()
+    P = ctypes.c_void_p
+    lib.et_linear_1x16_fwd.argtypes = [P, P, P, ctypes.c_int, P, P, P] + [ctypes.c_int] * 4 + [P]
+    args = lambda T: (P(0x1000), P(0x2000), P(0x3000), 4, None, P(0x4000), P(0x5000), T, 64, 64, 0, None)
+    assert lib.et_linear_1x16_fwd(*args(65535 * 128 + 1)) == -3
