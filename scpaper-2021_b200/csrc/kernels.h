@@ -84,6 +84,10 @@ int launch_linear_tile_rows(const int* row_ptr, const int* row_off, const __half
                             const __half* bias, const __half* X, __half* Y, int T, int in, int out,
                             int act, cudaStream_t stream);
 
+// The CSR Linear on the CUDA cores, for almost empty weights (linear_misc.cu).  Arguments already checked.
+int launch_linear_csr_rows(const int* indptr, const int* indices, const __half* data, const __half* bias,
+                           const __half* X, __half* Y, int T, int in, int out, int act, cudaStream_t stream);
+
 // The packed tile-CSR Linear with weights expanded to dense operand tiles in shared memory; see
 // linear_expand.cu.
 int launch_linear_expand_packed(const uint32_t* pk_mask, const int* pk_off, const __half* pk_tiles,

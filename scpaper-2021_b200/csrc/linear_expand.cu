@@ -569,14 +569,14 @@ int launch_bn(const CUtensorMap& tmX, ExpandArgs& a, cudaStream_t stream) {
                : ET_ERR_CUDA;
 }
 
+struct ExpandPlan {
+    int bn;
+    long panels, waves, cycles;
+};
+
+// Fills in a.mb, a.groups, a.ckb, a.nbuf and a.na.
 template <int FMT>
-int launch_expand(ExpandArgs a, cudaStream_t stream) {
-    CUtensorMap tmX;
-    int st = encode_operand(&tmX, a.X, a.in, a.T, a.in, BM);
-    if (st != ET_OK) return st;
-    a.err_word = device_error_word();
-    if (!a.err_word) return ET_ERR_NO_DEVICE;
-    a.vec_store = (a.out % 8 == 0 && aligned16(a.Y)) ? 1 : 0;
+ExpandPlan plan_expand(ExpandArgs& a) {
     const int sms = sm_count() > 0 ? sm_count() : 148;
     const long tblocks = (a.T + BM - 1) / BM;
     const int nkb = (a.in + BK - 1) / BK;
@@ -590,20 +590,18 @@ int launch_expand(ExpandArgs a, cudaStream_t stream) {
     // Token blocks per CTA: the count whose waves x time is least; a CTA costs about 4000 cycles of
     // set-up and epilogue besides its K blocks.
     const int mb_max = 512 / bn < X_MAX_MB ? 512 / bn : X_MAX_MB;
-    long best = -1;
+    long best = -1, best_waves = 0;
     for (int mb = 1; mb <= mb_max && mb <= tblocks; ++mb) {
         const long groups = (tblocks + mb - 1) / mb;
         const long waves = (panels(bn) * groups + sms - 1) / sms;
         const long cost = waves * (4000 + static_cast<long>(mb) * (nkb * (bn == 128 ? 256 : 240) + 600));
         if (best < 0 || cost < best) {
             best = cost;
+            best_waves = waves;
             a.mb = mb;
             a.groups = static_cast<int>(groups);
         }
     }
-    int cols = 32;
-    while (cols < a.mb * bn) cols <<= 1;
-    a.tmem_cols = cols;
     if (FMT == FMT_CSRM) {
         const int fit = X_CSR_BYTES / (bn * 128);
         a.ckb = nkb < fit ? nkb : fit;
@@ -614,6 +612,41 @@ int launch_expand(ExpandArgs a, cudaStream_t stream) {
         a.nbuf = X_MAX_B;
         a.na = X_MAX_A;
     }
+    return ExpandPlan{bn, panels(bn), best_waves, best};
+}
+
+// Whether the kernel whose work follows the stored values (linear_misc.cu) is expected to be faster than
+// expanding them, which costs a dense product whatever is stored.  Both times in microseconds, fitted to B200
+// runs at 512 -> 512, 768 -> 768, 1024 -> 3072, 3072 -> 768 and 4096 -> 1024, 1 to 8192 tokens and 0 to 50 %
+// stored: the faster one is chosen, or one within 20 % of it.  By values, by expansion: 3072 -> 768 at 2048 tokens
+// 0.1 % stored 10.0 / 22.2, 0.5 % 22.5 / 25.2, 1 % 39.8 / 28.9; 1024 -> 3072 at 8192 tokens none stored 19 / 70,
+// 0.1 % 39 / 72, 0.5 % 93 / 73; 4096 -> 1024 at 8192 tokens 0.1 % 50 / 113, 0.5 % 148 / 119.
+int g_csr_rows = -1;  // test hook: -1 = automatic, 0 = never, 1 = always
+bool csr_rows_pay(ExpandArgs a, int nnz) {
+    if (g_csr_rows >= 0) return g_csr_rows != 0;
+    const ExpandPlan p = plan_expand<FMT_CSRM>(a);
+    const double sms = sm_count() > 0 ? sm_count() : 148;
+    const double buffers = ((a.in + BK - 1) / BK + a.ckb - 1) / a.ckb;  // each waits for the one before it
+    const double expand =
+        0.3 + p.cycles / 1650.0 + p.waves * (1.9 * (buffers - 1) + 0.0012 * buffers * nnz / p.panels);
+    const double ctas = a.T / 8.0 / sms;  // per SM
+    const double rows = 2.1 + 0.0025 * a.out + 0.0022 * (nnz < a.out ? nnz : a.out) +
+                        2.0 * a.T * a.in / 5e6 + 0.0007 * (ctas > 1.2 ? ctas : 1.2) * nnz;
+    return rows < expand;
+}
+
+template <int FMT>
+int launch_expand(ExpandArgs a, cudaStream_t stream) {
+    CUtensorMap tmX;
+    int st = encode_operand(&tmX, a.X, a.in, a.T, a.in, BM);
+    if (st != ET_OK) return st;
+    a.err_word = device_error_word();
+    if (!a.err_word) return ET_ERR_NO_DEVICE;
+    a.vec_store = (a.out % 8 == 0 && aligned16(a.Y)) ? 1 : 0;
+    const int bn = plan_expand<FMT>(a).bn;
+    int cols = 32;
+    while (cols < a.mb * bn) cols <<= 1;
+    a.tmem_cols = cols;
     if (bn == 32) return launch_bn<FMT, 32>(tmX, a, stream);
     if (bn == 64) return launch_bn<FMT, 64>(tmX, a, stream);
     return launch_bn<FMT, FMT == FMT_CSRM ? 64 : 128>(tmX, a, stream);
@@ -685,7 +718,23 @@ int et_linear_csr_fwd(const int32_t* indptr, const int32_t* indices, const et_ha
     a.in = in;
     a.out = out;
     a.act = act;
+    if (et::csr_rows_pay(a, nnz))
+        return et::launch_linear_csr_rows(a.idx0, a.idx1, a.data, a.bias, a.X, a.Y, T, in, out, act,
+                                          static_cast<cudaStream_t>(stream));
     return et::launch_expand<et::FMT_CSRM>(a, static_cast<cudaStream_t>(stream));
 }
+
+#ifdef ET_TEST_HOOKS
+// Test hook: the CSR product by stored values: -1 = automatic, 0 = never, 1 = always.
+void et_debug_set_csr_rows(int mode) { et::g_csr_rows = mode; }
+// Test hook: 1 when that product is chosen for the size.
+int et_debug_csr_rows_pay(int T, int in, int out, int nnz) {
+    et::ExpandArgs a = {};
+    a.T = T;
+    a.in = in;
+    a.out = out;
+    return et::csr_rows_pay(a, nnz) ? 1 : 0;
+}
+#endif  // ET_TEST_HOOKS
 
 }  // extern "C"

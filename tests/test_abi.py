@@ -192,3 +192,14 @@ def test_1x16_refuses_more_than_65535_token_blocks(et):
     lib.et_linear_1x16_fwd.argtypes = [P, P, P, ctypes.c_int, P, P, P] + [ctypes.c_int] * 4 + [P]
     args = lambda T: (P(0x1000), P(0x2000), P(0x3000), 4, None, P(0x4000), P(0x5000), T, 64, 64, 0, None)
     assert lib.et_linear_1x16_fwd(*args(65535 * 128 + 1)) == -3
+
+
+def test_csr_plan_follows_the_stored_values(et):
+    """Almost empty weights take the kernel whose work follows what is stored (it was 2 to 5 times as fast there),
+    others the expanded tensor-core product, and nothing in between switches back."""
+    pays = et.lib().et_debug_csr_rows_pay
+    for T, inn, out in ((8192, 1024, 3072), (2048, 3072, 768), (128, 3072, 768), (8192, 4096, 1024), (8192, 768, 768)):
+        total = inn * out
+        chosen = [pays(T, inn, out, int(total * f)) for f in (0.0, 0.001, 0.01, 0.03, 0.1, 0.5)]
+        assert chosen[0] == chosen[1] == 1 and chosen[3:] == [0, 0, 0], (T, inn, out, chosen)
+        assert chosen == sorted(chosen, reverse=True)

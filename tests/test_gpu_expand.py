@@ -140,8 +140,13 @@ def test_an_infinity_reaches_only_outputs_that_store_a_weight_for_it(et, orc, cu
         _same_with_infinities(y, orc.linear_1x16(xf, ti, ri, dv, out, b, 0), "1x16")
         wc = w * (et.synth.uniform(75, 7, out * inn).reshape(out, inn) >= 0.9)
         ip, ix, dc = et.synth.dense_to_csr(wc)
-        y = et.linear_csr(d(x), d(ip), d(ix), d(dc), out, d(b), 0)
-        _same_with_infinities(y, orc.linear_csr(xf, ip, ix, dc, out, b, 0), "csr")
+        for mode in (0, 1):  # expanded, by stored values
+            et.lib().et_debug_set_csr_rows(ctypes.c_int(mode))
+            try:
+                y = et.linear_csr(d(x), d(ip), d(ix), d(dc), out, d(b), 0)
+            finally:
+                et.lib().et_debug_set_csr_rows(ctypes.c_int(-1))
+            _same_with_infinities(y, orc.linear_csr(xf, ip, ix, dc, out, b, 0), f"csr {mode}")
         wt = et.synth.prune_tiles(w, 75, 4, 0.8)
         rp, ro, tiles = et.synth.dense_to_tile(wt)
         ref = orc.linear_tile(xf, rp, ro, tiles, out, b, 0)
@@ -191,3 +196,24 @@ assert (y == 400).all() and et.device_error() == 0
 """ % ROOT
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=180)
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+@pytest.mark.parametrize("T,inn,out,sparsity", [(1, 16, 16, 0.9), (9, 24, 5, 0.5), (77, 1000, 203, 0.97),
+                                                (130, 8192, 40, 0.999), (300, 1024, 515, 1.0)])
+def test_csr_by_stored_values(et, orc, cuda, T, inn, out, sparsity):
+    """The kernel for almost empty weights, at its remainders (8 tokens, 256 features) and its widest row."""
+    import ctypes
+    x, w, b = _case(et, 78, T, inn, out)
+    w = w * (et.synth.uniform(78, 7, out * inn).reshape(out, inn) >= sparsity)
+    ip, ix, data = et.synth.dense_to_csr(w)
+    n = len(ix)
+    ref = orc.linear_csr(x, ip, ix, data, out, b, 1)
+    for mode in (1, 0, -1):
+        et.lib().et_debug_set_csr_rows(ctypes.c_int(mode))
+        try:
+            y = et.linear_csr(_dev(x, cuda), _dev(ip, cuda), _dev(ix, cuda) if n else None,
+                              _dev(data, cuda) if n else None, out, _dev(b, cuda), 1)
+        finally:
+            et.lib().et_debug_set_csr_rows(ctypes.c_int(-1))
+        assert et.device_error() == 0
+        _check(y, ref, f"csr by values {T}x{inn}x{out} mode {mode}")
