@@ -95,6 +95,13 @@ __global__ void pack_tiles_kernel(const uint4* __restrict__ src, const int* __re
 int g_tile_wide = -1;  // test hook: -1 = automatic, 0 = one panel per CTA, 1 = two panels per CTA
 
 namespace {
+// Whether packed weights run on the expanding kernel (the reasons stand where it is called).
+bool tile_packed_expands(int T, int in, int out, int nnz_tiles) {
+    const long out_tiles = static_cast<long>((out + TBN - 1) / TBN) * ((T + TBM - 1) / TBM);
+    const long all = static_cast<long>(in / 16) * (out / 16);
+    return in >= 2048 && 2 * out_tiles <= (sm_count() > 0 ? sm_count() : 148) && 100L * nnz_tiles > 3 * all;
+}
+
 int launch_tile_common(bool packed, const int* row_ptr, const int* row_off, const uint32_t* pk_mask,
                        const int* pk_off, const __half* tiles, int nnz_tiles, const __half* bias,
                        const __half* X, __half* Y, int T, int in, int out, int act,
@@ -125,10 +132,11 @@ int launch_tile_common(bool packed, const int* row_ptr, const int* row_off, cons
     // B200 at 80 / 90 / 95 % sparsity, this kernel against that: 3072 -> 768 at 1000 tokens (48 tiles) 18.4 / 16.5 /
     // 14.1 against 13.8 / 13.7 / 13.5 us, 4096 -> 1024 at 1000 (64 tiles) 24.6 / 21.0 / 18.7 against 17.0 us, 2048 -> 512
     // at 2048 (64 tiles) 14.0 / 12.7 / 11.1 against 10.3 us; with 96 tiles (3072 -> 768 at 2048) 19.7 / 17.4 / 14.9
-    // against 17.9 / 17.0 / 16.6 us, and 768-wide K gains nothing.
-    const long out_tiles = static_cast<long>((out + TBN - 1) / TBN) * ((T + TBM - 1) / TBM);
-    if (packed && (tile_packed_mode() == 2 || (tile_packed_mode() < 0 && g_tile_wide < 0 && in >= 2048 &&
-                                               2 * out_tiles <= (sm_count() > 0 ? sm_count() : 148))))
+    // against 17.9 / 17.0 / 16.6 us, and 768-wide K gains nothing.  This kernel's time follows what is stored, that
+    // one's does not: at 97 / 99 / 99.5 % 3072 -> 768 takes 12.4 / 10.3 / 9.7 against 12.9 us at 1000 tokens, and
+    // 4096 -> 1024 17.0 / 13.2 / 12.3 against 16.3 us.
+    if (packed && (tile_packed_mode() == 2 || (tile_packed_mode() < 0 && g_tile_wide < 0 &&
+                                               tile_packed_expands(T, in, out, nnz_tiles))))
         return launch_linear_expand_packed(pk_mask, pk_off, tiles, bias, X, Y, T, in, out, act, stream);
 
     CUtensorMap tmX, tmW, tmY;
@@ -232,6 +240,10 @@ int launch_linear_tile_packed(const int* row_ptr, const uint32_t* pk_mask, const
 extern "C" {
 
 #ifdef ET_TEST_HOOKS
+// Test hook: 1 when packed weights of this size run on the expanding kernel.
+int et_debug_tile_packed_expands(int T, int in, int out, int nnz_tiles) {
+    return et::tile_packed_expands(T, in, out, nnz_tiles) ? 1 : 0;
+}
 // Test hook: -1 = automatic, 0 = one panel per CTA, 1 = two panels per CTA (packed weights).
 void et_debug_set_tile_wide(int mode) { et::g_tile_wide = mode; }
 // Test hook: 1 = tile-CSR arrays run on the warp-level kernel, 0 = on the tcgen05 one (default).

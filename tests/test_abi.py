@@ -203,3 +203,13 @@ def test_csr_plan_follows_the_stored_values(et):
         chosen = [pays(T, inn, out, int(total * f)) for f in (0.0, 0.001, 0.01, 0.03, 0.1, 0.5)]
         assert chosen[0] == chosen[1] == 1 and chosen[3:] == [0, 0, 0], (T, inn, out, chosen)
         assert chosen == sorted(chosen, reverse=True)
+
+
+def test_almost_empty_packed_tiles_stay_on_the_kernel_that_follows_them(et):
+    """The expanding kernel takes long K with few output tiles, but not where hardly a tile is stored: its time
+    does not fall with them."""
+    expands = et.lib().et_debug_tile_packed_expands
+    for T, inn, out in ((1, 3072, 768), (1000, 3072, 768), (1000, 4096, 1024), (128, 2048, 512)):
+        total = (inn // 16) * (out // 16)
+        assert [expands(T, inn, out, int(total * f)) for f in (0.2, 0.1, 0.05, 0.01, 0.001)] == [1, 1, 1, 0, 0]
+    assert expands(8192, 3072, 768, 4608) == 0 and expands(128, 768, 3072, 4608) == 0
