@@ -820,14 +820,21 @@ int pick_tall(int M, int N, int K) {
 
 int g_force_narrow = -1;  // test hook: -1 = automatic, 0 = never, 32 / 64 = always that width
 
-// Width of the one-tile-per-CTA kernel for few output tiles (gemm_narrow.cu), or 0.
+// Width of the one-tile-per-CTA kernel for few output tiles (gemm_narrow.cu), or 0.  With up to half a row
+// block of tokens every CTA reads the same few lines of X, and the more CTAs the longer that takes: 3072 -> 768
+// (24 tiles of 32) 8.6 us against 10.0 for 128-wide tiles at 1 token, but 768 -> 3072 (96) 5.8 against 4.4,
+// 1024 -> 4096 (128) 9.9 against 6.0 and 3072 -> 3072 20.3 against 10.9; in 64-wide tiles 1024 -> 2048 (32) takes
+// 4.7 against 5.0 and 768 -> 3072 (48) 4.4.  At 32 tokens 48 to 64 of these are ahead again (1024 -> 3072 4.9
+// against 5.3, 3072 -> 4096 9.0 against 10.6), above 64 tokens the narrowest are.
 int pick_narrow(int M, int N) {
     if (g_force_narrow >= 0) return g_force_narrow;
     if (g_force_bn != 0 || g_force_persist >= 0 || g_force_pair > 0 || g_force_tall > 0) return 0;
     const long sms = sm_count() > 0 ? sm_count() : 148;
     const long mt = (M + BM - 1) / BM;
-    if (mt * ((N + 31) / 32) <= sms) return 32;
-    if (mt * ((N + 63) / 64) <= sms) return 64;
+    const long n32 = (N + 31) / 32, n64 = (N + 63) / 64;
+    if (M <= 64) return n32 <= 32 ? 32 : (n64 <= (M < 32 ? 36 : sms) ? 64 : 0);
+    if (mt * n32 <= sms) return 32;
+    if (mt * n64 <= sms) return 64;
     return 0;
 }
 
@@ -1039,6 +1046,8 @@ void et_debug_set_gemm_max_ctas(int n) { et::gemm_set_max_ctas(n); }
 void et_debug_force_gemm_tall(int mode) { et::gemm_force_tall(mode); }
 // Test hook: -1 = automatic, 0 = single-CTA kernels only, 128 / 256 = CTA-pair tiles of that width.
 void et_debug_force_gemm_pair(int mode) { et::gemm_force_pair(mode); }
+// Test hook: the width chosen for the size.
+int et_debug_gemm_narrow_width(int M, int N) { return et::pick_narrow(M, N); }
 // Test hook: -1 = automatic, 0 = never, 32 / 64 = one 128-row tile of that width per CTA.
 void et_debug_force_gemm_narrow(int mode) { et::gemm_force_narrow(mode); }
 // Test hook: -1 = automatic, 0 = one tile per CTA, 1 = persistent CTAs.

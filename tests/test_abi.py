@@ -213,3 +213,15 @@ def test_almost_empty_packed_tiles_stay_on_the_kernel_that_follows_them(et):
         total = (inn // 16) * (out // 16)
         assert [expands(T, inn, out, int(total * f)) for f in (0.2, 0.1, 0.05, 0.01, 0.001)] == [1, 1, 1, 0, 0]
     assert expands(8192, 3072, 768, 4608) == 0 and expands(128, 768, 3072, 4608) == 0
+
+
+def test_narrow_gemm_tiles_with_few_tokens(et):
+    """Tiles of the GEMM for few output tiles: with up to 64 tokens all CTAs read the same lines of X, so wide
+    outputs must not be cut into a hundred of them (1024 -> 4096 took 9.9 us for 6.0 at one token)."""
+    width = et.lib().et_debug_gemm_narrow_width
+    assert [width(1, n) for n in (512, 768, 1024, 2048, 2304, 3072, 4096)] == [32, 32, 32, 64, 64, 0, 0]
+    assert [width(31, n) for n in (1024, 2304, 3072)] == [32, 64, 0]
+    assert [width(32, n) for n in (1024, 2304, 3072, 4096)] == [32, 64, 64, 64]
+    assert [width(64, n) for n in (768, 3072)] == [32, 64]
+    assert [width(65, n) for n in (768, 3072, 4096)] == [32, 32, 32]
+    assert width(385, 768) == 32 and width(128 * 12, 768) == 64 and width(128 * 13, 768) == 0

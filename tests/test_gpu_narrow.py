@@ -20,7 +20,8 @@ def _dev(a, cuda):
 
 
 @pytest.mark.parametrize("T,inn,out,act", [(1, 16, 16, 0), (128, 768, 768, 0), (129, 80, 144, 2),
-                                           (300, 1040, 1008, 1), (385, 3072, 72, 2), (64, 64, 3072, 2)])
+                                           (300, 1040, 1008, 1), (385, 3072, 72, 2), (64, 64, 3072, 2),
+                                           (31, 256, 3072, 0), (33, 1024, 2320, 2)])
 def test_narrow_tiles_match_wide_ones(et, cuda, T, inn, out, act):
     import torch
     x = _dev(et.synth.normal_fast(81, 1, (T, inn), 1.0), cuda)
