@@ -825,14 +825,16 @@ int g_force_narrow = -1;  // test hook: -1 = automatic, 0 = never, 32 / 64 = alw
 // (24 tiles of 32) 8.6 us against 10.0 for 128-wide tiles at 1 token, but 768 -> 3072 (96) 5.8 against 4.4,
 // 1024 -> 4096 (128) 9.9 against 6.0 and 3072 -> 3072 20.3 against 10.9; in 64-wide tiles 1024 -> 2048 (32) takes
 // 4.7 against 5.0 and 768 -> 3072 (48) 4.4.  At 32 tokens 48 to 64 of these are ahead again (1024 -> 3072 4.9
-// against 5.3, 3072 -> 4096 9.0 against 10.6), above 64 tokens the narrowest are.
+// against 5.3, 3072 -> 4096 9.0 against 10.6).  At 64 tokens 72 of 32 columns are (1024 -> 2304 4.2 against 4.7 in
+// 64-wide tiles) but not 96 (768 -> 3072 5.3 against 4.2), above 64 tokens all that fit.
 int pick_narrow(int M, int N) {
     if (g_force_narrow >= 0) return g_force_narrow;
     if (g_force_bn != 0 || g_force_persist >= 0 || g_force_pair > 0 || g_force_tall > 0) return 0;
     const long sms = sm_count() > 0 ? sm_count() : 148;
     const long mt = (M + BM - 1) / BM;
     const long n32 = (N + 31) / 32, n64 = (N + 63) / 64;
-    if (M <= 64) return n32 <= 32 ? 32 : (n64 <= (M < 32 ? 36 : sms) ? 64 : 0);
+    if (M <= 32) return n32 <= 32 ? 32 : (n64 <= (M < 32 ? 36 : sms) ? 64 : 0);
+    if (M <= 64) return n32 <= 72 ? 32 : (n64 <= sms ? 64 : 0);
     if (mt * n32 <= sms) return 32;
     if (mt * n64 <= sms) return 64;
     return 0;

@@ -222,6 +222,7 @@ def test_narrow_gemm_tiles_with_few_tokens(et):
     assert [width(1, n) for n in (512, 768, 1024, 2048, 2304, 3072, 4096)] == [32, 32, 32, 64, 64, 0, 0]
     assert [width(31, n) for n in (1024, 2304, 3072)] == [32, 64, 0]
     assert [width(32, n) for n in (1024, 2304, 3072, 4096)] == [32, 64, 64, 64]
-    assert [width(64, n) for n in (768, 3072)] == [32, 64]
+    assert [width(64, n) for n in (768, 2304, 3072)] == [32, 32, 64]
+    assert [width(33, n) for n in (2304, 2320)] == [32, 64]
     assert [width(65, n) for n in (768, 3072, 4096)] == [32, 32, 32]
     assert width(385, 768) == 32 and width(128 * 12, 768) == 64 and width(128 * 13, 768) == 0
