@@ -120,10 +120,19 @@ int make_tensor_map(CUtensorMap* map, CUtensorMapDataType dtype, const void* bas
         if (strides_bytes[i] % 16 != 0) return ET_ERR_ALIGNMENT;
         gstrides[i] = strides_bytes[i];
     }
-    CUresult r = encode(map, dtype, static_cast<cuuint32_t>(rank),
-                          const_cast<void*>(base), gdims, gstrides, gbox, estr,
-                          CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    auto make = [&]() {
+        return encode(map, dtype, static_cast<cuuint32_t>(rank), const_cast<void*>(base), gdims, gstrides, gbox,
+                      estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    };
+    CUresult r = make();
+    if (r == CUDA_ERROR_INVALID_CONTEXT) {
+        // a thread that has made no runtime call that needs the device's context has none yet, and this is a
+        // driver call
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess) return ET_ERR_CUDA;
+        r = make();
+    }
     return r == CUDA_SUCCESS ? ET_OK : ET_ERR_CUDA;
 }
 }  // namespace
