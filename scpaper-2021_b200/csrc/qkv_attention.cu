@@ -43,6 +43,7 @@ constexpr int QA_ATOM = 128 * 128;               // 128 rows x 64 fp16
 constexpr int QA_STAGE = QA_ATOM + 3 * 64 * 128; // X block + three weight slices = 40 KB
 constexpr int QA_MISC = 256 + 192 * 4 + 6 * 128 * 4;
 constexpr int QA_MAX_STAGES = 5;
+constexpr int QA_DEEP_MASK_BYTES = 22 * 1024;
 __host__ __device__ constexpr int qa_smem(int stages) { return stages * QA_STAGE + QA_MISC + 1024; }
 constexpr int QA_TMEM = 256;
 static_assert(2 * QA_STAGE == 5 * QA_ATOM, "two stages must hold Q, K, V and two atoms of P");
@@ -414,6 +415,20 @@ bool qkv_attention_applies(int seq, int nhead, int kdim, int vdim) {
     return seq > 0 && seq <= 128 && nhead > 0 && kdim == nhead * 64 && vdim == nhead * 64;
 }
 
+// Whether the projection takes the five-stage ring, one CTA to an SM: with a CTA per SM to spare, but not where
+// an additive mask no longer fits the L1 cache that 200 KB of shared memory leave (a thread reads its mask row two
+// bytes at a time).  Two stages against five, 12 heads: 1 x 100 tokens (a mask of 20 KB) 14.5 / 12.8 us, 1 x 112
+// 13.7 / 18.1, 4 x 120 15.5 / 20.2, 1 x 128 17.8 / 21.9.  Rows of 128 positions, 256 bytes apart, miss either way
+// once there are many CTAs: 4 x 128 23.4 / 22.7, 9 x 128 27.6 / 23.7 us.
+int g_qkv_deep = -1;  // test hook: -1 = automatic, 0 / 1 = two / five stages
+bool qkv_attention_deep(int seq, int nhead, int batch, int mask_kind) {
+    if (g_qkv_deep >= 0) return g_qkv_deep != 0;
+    const long ctas = static_cast<long>(nhead) * batch;
+    if (mask_kind == ET_MASK_ADDITIVE && 2 * seq * seq > QA_DEEP_MASK_BYTES && (seq != 128 || ctas <= 32))
+        return false;
+    return ctas <= (sm_count() > 0 ? sm_count() : 148);
+}
+
 // Z[b, :, h * 64 ..] = softmax(Q_h K_h^T * scale + mask) V_h with [Q | K | V] = X Wqkv^T + b.
 int launch_qkv_attention(const __half* X, const __half* Wqkv, const __half* bqkv, __half* Z,
                          int batch, int seq, int hidden, int nhead, int kdim, int vdim, int ldz,
@@ -473,7 +488,7 @@ int launch_qkv_attention(const __half* X, const __half* Wqkv, const __half* bqkv
                    ? ET_OK
                    : ET_ERR_CUDA;
     };
-    const bool deep = static_cast<long>(nhead) * batch <= sm_count();
+    const bool deep = qkv_attention_deep(seq, nhead, batch, mask_kind);
     auto by_depth = [&](auto mask, const QkvAttnArgs& args) -> int {
         constexpr int M = decltype(mask)::value;
         return deep ? go(qkv_attention_kernel<M, QA_MAX_STAGES>, 4 + M, qa_smem(QA_MAX_STAGES), args)
@@ -500,6 +515,15 @@ int launch_qkv_attention(const __half* X, const __half* Wqkv, const __half* bqkv
 }  // namespace et
 
 extern "C" {
+
+#ifdef ET_TEST_HOOKS
+// Test hook: stages of the projection's ring: -1 = automatic, 0 = two, 1 = five.
+void et_debug_set_qkv_deep(int mode) { et::g_qkv_deep = mode; }
+// Test hook: 1 when five are chosen for the size.
+int et_debug_qkv_deep(int seq, int nhead, int batch, int mask_kind) {
+    return et::qkv_attention_deep(seq, nhead, batch, mask_kind) ? 1 : 0;
+}
+#endif  // ET_TEST_HOOKS
 
 int et_qkv_attention_fwd(const et_half* X, const et_half* Wqkv, const et_half* bqkv, et_half* Z,
                          int batch, int seq, int hidden, int nhead, int kdim, int vdim,

@@ -226,3 +226,12 @@ def test_narrow_gemm_tiles_with_few_tokens(et):
     assert [width(33, n) for n in (2304, 2320)] == [32, 64]
     assert [width(65, n) for n in (768, 3072, 4096)] == [32, 32, 32]
     assert width(385, 768) == 32 and width(128 * 12, 768) == 64 and width(128 * 13, 768) == 0
+
+
+def test_depth_of_the_fused_projection_ring(et):
+    """Five stages where every CTA has an SM to itself, but not beside an additive mask that they would push out
+    of the L1 cache (1 x 128 tokens, 12 heads, had gone from 18.4 to 22.2 us)."""
+    deep = et.lib().et_debug_qkv_deep
+    assert [deep(128, 12, b, 0) for b in (1, 12, 13)] == [1, 1, 0]
+    assert [deep(s, 12, 1, 3) for s in (1, 100, 106, 107, 127, 128)] == [1, 1, 1, 0, 0, 0]
+    assert [deep(128, 12, b, 3) for b in (2, 3, 12, 13)] == [0, 1, 1, 0]
