@@ -98,7 +98,7 @@ def test_packed_tiles(et, orc, cuda, T, inn, out, sparsity):
         finally:
             L.et_debug_set_tile_persist(ctypes.c_int(-1))
     _check(ys[0], orc.linear_dense(x, w, b, 2), f"packed {T}x{inn}x{out} s={sparsity}")
-    # the products of absent tiles add exact zeros: the same bits
+    # on finite activations the products of absent tiles add exact zeros: the same bits
     assert torch.equal(ys[0], ys[1])
 
 

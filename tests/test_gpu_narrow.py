@@ -20,7 +20,7 @@ def _dev(a, cuda):
 
 
 @pytest.mark.parametrize("T,inn,out,act", [(1, 16, 16, 0), (128, 768, 768, 0), (129, 80, 144, 2),
-                                           (300, 1040, 1008, 1), (385, 3072, 72, 2), (64, 64, 3072, 2),
+                                           (300, 1040, 1008, 1), (385, 3072, 80, 2), (64, 64, 3072, 2),
                                            (31, 256, 3072, 0), (33, 1024, 2320, 2)])
 def test_narrow_tiles_match_wide_ones(et, cuda, T, inn, out, act):
     import torch
@@ -32,12 +32,11 @@ def test_narrow_tiles_match_wide_ones(et, cuda, T, inn, out, act):
     try:
         for bn in (0, 32, 64):
             L.et_debug_force_gemm_narrow(ctypes.c_int(bn))
-            ys.append(et.linear_dense(x, w, b, act) if out % 16 == 0 else None)
+            ys.append(et.linear_dense(x, w, b, act))
             assert et.device_error() == 0
     finally:
         L.et_debug_force_gemm_narrow(ctypes.c_int(-1))
-    if out % 16 == 0:
-        assert torch.equal(ys[0], ys[1]) and torch.equal(ys[0], ys[2])
+    assert torch.equal(ys[0], ys[1]) and torch.equal(ys[0], ys[2])
 
 
 @pytest.mark.parametrize("batch,seq,hidden,nhead,ff", [
@@ -60,6 +59,16 @@ def test_layer_with_few_row_blocks(et, orc, cuda, batch, seq, hidden, nhead, ff)
     ref = orc.encoder_layer(x.astype(np.float32), w, batch, seq, nhead, 2, 2, None, vl)
     assert_close(y.float().cpu().numpy(), ref, f"layer {batch}x{seq}x{hidden}")
     assert torch.equal(y, stack.forward(_dev(x, cuda), et.MASK_PADDING, None, _dev(vl, cuda)))
+    # and with the fused or the plain Linear + LayerNorm in place of the K slices: the plain one rounds the product
+    # to fp16 before the LayerNorm
+    et.lib().et_debug_set_narrow_ln(ctypes.c_int(0))
+    try:
+        other = stack.forward(_dev(x, cuda), et.MASK_PADDING, None, _dev(vl, cuda))
+    finally:
+        et.lib().et_debug_set_narrow_ln(ctypes.c_int(-1))
+    assert et.device_error() == 0
+    assert_close(y.float().cpu().numpy(), other.float().cpu().numpy(), f"forms of {batch}x{seq}x{hidden}",
+                 rel_tol=1.5e-3)
 
 
 @pytest.mark.parametrize("batch,seq", [(1, 128), (5, 77)])
