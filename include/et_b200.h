@@ -189,15 +189,22 @@ int et_linear_col_noalloc_fwd(const int32_t* col_id, const et_half* cols, int nn
                               int out, int act, et_stream stream);
 
 /* 1x16-vector weights: tile_idx[(out/16) * (in/16 + 1)], row_idx[nvec], data[nvec][16]
- * (mat_type/mat1x16/mat1x16.h:9-15).  Stands in for Linear<mat1x16>::forward
+ * (mat_type/mat1x16/mat1x16.h:9-15), the row_idx of a part ascending and without repetition
+ * (et_validate_1x16).  Stands in for Linear<mat1x16>::forward
  * (Linear/SPMM1x16.cu:89-115, whose body the reference leaves empty; the intended
- * product of :56-83 is computed). */
+ * product of :56-83 is computed).  Like every weight, the arrays must be complete (stream
+ * synchronised) before the first call that uses them: they are fetched before the kernel waits
+ * for its predecessors on the stream. */
 int et_linear_1x16_fwd(const int32_t* tile_idx, const int32_t* row_idx, const et_half* data,
                        int nvec, const et_half* bias, const et_half* X, et_half* Y, int T, int in,
                        int out, int act, et_stream stream);
 
-/* CSR weights W[out, in].  Stands in for Linear<csr_mat>::forward (Linear/cusp.cu:23-50:
- * cuSPARSE SpMM + bias pass). */
+/* CSR weights W[out, in]; the entries of a row in any order, values of a repeated column add up.
+ * The arrays must be complete before the first call that uses them, as those of
+ * et_linear_1x16_fwd.  Stands in for Linear<csr_mat>::forward (Linear/cusp.cu:23-50:
+ * cuSPARSE SpMM + bias pass).
+ * In all three sparse formats an infinite or NaN activation reaches only the outputs that store a
+ * weight (a vector, a tile) for it. */
 int et_linear_csr_fwd(const int32_t* indptr, const int32_t* indices, const et_half* data,
                       int nnz, const et_half* bias, const et_half* X, et_half* Y, int T, int in,
                       int out, int act, et_stream stream);

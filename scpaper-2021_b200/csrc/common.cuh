@@ -532,18 +532,7 @@ __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols
                  : "memory");
 }
 // D[tmem of both CTAs] (+)= A . B over the pair (M = 256); issued by ONE thread of the leader.
-__device__ __forceinline__ void mma_f16_ss_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                                uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
-        "}\n"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// (operands given by their descriptors' low words, as mma_f16_ss_k128)
+// Operands given by their descriptors' low words, as mma_f16_ss_k128.
 __device__ __forceinline__ void mma_f16_ss_pair_k128(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo,
                                                      uint32_t idesc, uint32_t accumulate) {
     asm volatile(
